@@ -1555,7 +1555,10 @@ __device__ __forceinline__ void wall_friction(const DevP& P, float& vx, float& v
 // then the arithmetic in ascending row order, so the loads of a batch overlap instead of forming one dependent
 // chain per neighbour. Entries past the row's end address the particle itself (a harmless load) and are skipped.
 // NB is a template parameter of every neighbour loop (the gathers a thread keeps in flight); the autotuner picks it
-// per kernel among NB_CHOICES, NB_DEFAULT otherwise.
+// per kernel among NB_CHOICES, NB_DEFAULT otherwise. The loops that read (entry, F) rows load each batch while the one
+// before it is gathered: the rows come from HBM, the gathers mostly from L1, so the row's latency was the longer one
+// (Jacobi 208.9 -> 200.7 us, acceleration 148.6 -> 140.1 us on 160 worlds of 2,000 to 32,000 particles; 123.7 -> 120.8
+// and 81.6 -> 79.0 us on the 1M dam break, where the L1's gathers bound them).
 constexpr int NB_DEFAULT = 8;
 
 // Rows are streamed once per kernel (evict-first loads) so that the gathered particle arrays keep L1 and L2.
@@ -1577,6 +1580,16 @@ __device__ __forceinline__ void load_row_batch_f(const DevP& P, int p, int c, in
     int2 e = (k + u < c) ? __ldcs(row + (size_t)(k + u) * P.n) : make_int2(p, 0);
     j[u] = e.x;
     f[u] = __int_as_float(e.y);
+  }
+}
+
+// The batch loaded ahead becomes the current one.
+template <int NB>
+__device__ __forceinline__ void next_batch(int (&j)[NB], float (&f)[NB], const int (&jn)[NB], const float (&fn)[NB]) {
+#pragma unroll
+  for (int u = 0; u < NB; ++u) {
+    j[u] = jn[u];
+    f[u] = fn[u];
   }
 }
 
@@ -1647,42 +1660,11 @@ __global__ void __launch_bounds__(BLOCK, 5) k_density_alpha(DevP P) {
 
 // --------------------------------------------------------------------------------------------- solve start
 // pressure.py:196-261
-template <int NBX>
-__global__ void __launch_bounds__(BLOCK) k_solve_init(DevP P) {
-  constexpr int NB = NBX & NB_MASK;
-  constexpr bool MS = (NBX & MS_FLAG) != 0;
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.nfw[0]) return;
-  float4 xi = P.pos[p];
-  float4 vi = P.vel[p];
-  float inv_r0 = 1.0f / vi.w;
-  float rate = 0.0f;
-  int c = P.cnt[p];
-  for (int k = 0; k < c; k += NB) {
-    int j[NB];
-    float fb[NB];
-    load_row_batch_f(P, p, c, k, j, fb);
-    float4 xb[NB], vb[NB];
-#pragma unroll
-    for (int u = 0; u < NB; ++u) {
-      xb[u] = P.pos[j[u]];
-      vb[u] = P.vel[j[u]];
-    }
-#pragma unroll
-    for (int u = 0; u < NB; ++u) {
-      if (k + u >= c) break;
-      float4 xj = xb[u], vj = vb[u];
-      float rx = xi.x - xj.x, ry = xi.y - xj.y, rz = xi.z - xj.z;
-      float aF = (xj.w * inv_r0) * fb[u];
-      rate = ADF_FMA(aF, dotf(vi.x - vj.x, vi.y - vj.y, vi.z - vj.z, rx, ry, rz), rate);
-    }
-  }
-  for_slots<MS>(P, p, [&](int, size_t o) {
-    const float4 sg = P.slot_g[o], vb = P.slot_vb[o];
-    rate = rate + dotf(vi.x - vb.x, vi.y - vb.y, vi.z - vb.z, sg.x, sg.y, sg.z);
-  });
+// The source, the lower bound and the plain start of particle p from its divergence `rate` (and the warm-start
+// features, when they are recorded).
+__device__ __forceinline__ void solve_start(const DevP& P, int p, const float4& vi, float rate, float& kap, float& lb,
+                                            float& src) {
   const float dt = P.dt;
-  float kap, lb, s;
   if (P.mode == 0) {
     float kdv = 0.0f;
     if (P.two_sided) kdv = maxr((P.warm_den * minr(P.kd_s[p], (float)(2.5e-4))) / (dt * dt), 0.0f);
@@ -1696,17 +1678,17 @@ __global__ void __launch_bounds__(BLOCK) k_solve_init(DevP P) {
       r = 0.0f;
       lb = 0.0f;
     }
-    s = r;
+    src = r;
     kap = maxr((P.warm * minr(P.kv_s[p], 0.5f)) / dt, lb);
   } else {
     float ratio = P.ratio[p];
     float rs = ADF_FMA(dt, rate, ratio);
     if (ratio - 1.0f > P.relief) rs = ADF_FMA(dt, rate, 1.0f + P.relief);
-    s = rs;
+    src = rs;
     lb = 0.0f;
     kap = (P.warm * minr(P.kd_s[p], (float)(2.5e-4))) / (dt * dt);
   }
-  P.src[p] = s;
+  P.src[p] = src;
   P.lower[p] = lb;
   P.kappa[p] = kap;
   P.kr[p] = kap / vi.w;
@@ -1728,6 +1710,52 @@ __global__ void __launch_bounds__(BLOCK) k_solve_init(DevP P) {
     fr[2] = f2;
     fr[3] = f3;
   }
+}
+
+template <int NBX>
+__device__ __forceinline__ void solve_init_one(const DevP& P, int p) {
+  constexpr int NB = NBX & NB_MASK;
+  constexpr bool MS = (NBX & MS_FLAG) != 0;
+  float4 xi = P.pos[p];
+  float4 vi = P.vel[p];
+  float inv_r0 = 1.0f / vi.w;
+  float rate = 0.0f;
+  int c = P.cnt[p];
+  int jn[NB];
+  float fn[NB];
+  load_row_batch_f(P, p, c, 0, jn, fn);
+  for (int k = 0; k < c; k += NB) {
+    int j[NB];
+    float fb[NB];
+    next_batch<NB>(j, fb, jn, fn);
+    load_row_batch_f(P, p, c, k + NB, jn, fn);
+    float4 xb[NB], vb[NB];
+#pragma unroll
+    for (int u = 0; u < NB; ++u) {
+      xb[u] = P.pos[j[u]];
+      vb[u] = P.vel[j[u]];
+    }
+#pragma unroll
+    for (int u = 0; u < NB; ++u) {
+      if (k + u >= c) break;
+      float4 xj = xb[u], vj = vb[u];
+      float rx = xi.x - xj.x, ry = xi.y - xj.y, rz = xi.z - xj.z;
+      float aF = (xj.w * inv_r0) * fb[u];
+      rate = ADF_FMA(aF, dotf(vi.x - vj.x, vi.y - vj.y, vi.z - vj.z, rx, ry, rz), rate);
+    }
+  }
+  for_slots<MS>(P, p, [&](int, size_t o) {
+    const float4 sg = P.slot_g[o], vb = P.slot_vb[o];
+    rate = rate + dotf(vi.x - vb.x, vi.y - vb.y, vi.z - vb.z, sg.x, sg.y, sg.z);
+  });
+  float kap, lb, src;
+  solve_start(P, p, vi, rate, kap, lb, src);
+}
+
+template <int NBX>
+__global__ void __launch_bounds__(BLOCK) k_solve_init(DevP P) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < P.nfw[0]) solve_init_one<NBX>(P, p);
 }
 
 // The learned start of this solve: the plain start (the previous warm start scaled, in dt-free units) plus the
@@ -1981,10 +2009,14 @@ __device__ __forceinline__ void pressure_accel(const DevP& P, int p, float4 xi, 
   float ki = P.kr[p];
   ax = ay = az = 0.0f;
   int c = P.cnt[p];
+  int jn[NB];
+  float fn[NB];
+  src.template row<NB>(P, p, c, 0, jn, fn);
   for (int k = 0; k < c; k += NB) {
     int j[NB];
     float fb[NB];
-    src.template row<NB>(P, p, c, k, j, fb);
+    next_batch<NB>(j, fb, jn, fn);
+    src.template row<NB>(P, p, c, k + NB, jn, fn);
     float4 xb[NB];
     float kb[NB];
 #pragma unroll
@@ -2033,10 +2065,14 @@ __device__ __forceinline__ float accel_divergence(const DevP& P, int p, float in
   float4 ai = P.acc[p];
   float ar = 0.0f;
   int c = P.cnt[p];
+  int jn[NB];
+  float fn[NB];
+  src.template row<NB>(P, p, c, 0, jn, fn);
   for (int k = 0; k < c; k += NB) {
     int j[NB];
     float fb[NB];
-    src.template row<NB>(P, p, c, k, j, fb);
+    next_batch<NB>(j, fb, jn, fn);
+    src.template row<NB>(P, p, c, k + NB, jn, fn);
     float4 xb[NB], ab[NB];
 #pragma unroll
     for (int u = 0; u < NB; ++u) {
@@ -2059,11 +2095,8 @@ __device__ __forceinline__ float accel_divergence(const DevP& P, int p, float in
   return ar;
 }
 
-template <int NBX, class R = GlobalRows>
-__device__ __forceinline__ void jacobi_one(const DevP& P, int p, const R& src = R()) {
-  float r0 = P.vel[p].w;
-  float inv_r0 = 1.0f / r0;
-  float ar = accel_divergence<NBX>(P, p, inv_r0, src);
+// The update of kappa and the residual of particle p from Ar (ar).
+__device__ __forceinline__ void jacobi_update(const DevP& P, int p, float r0, float ar) {
   float kap = P.kappa[p];
   ar = ADF_FMA(-P.reg[p], kap, ar);
   const float dt = P.dt;
@@ -2084,6 +2117,12 @@ __device__ __forceinline__ void jacobi_one(const DevP& P, int p, const R& src = 
     e = e * dt;
   }
   P.err_orig[P.id_of[p]] = e;
+}
+
+template <int NBX, class R = GlobalRows>
+__device__ __forceinline__ void jacobi_one(const DevP& P, int p, const R& src = R()) {
+  const float r0 = P.vel[p].w;
+  jacobi_update(P, p, r0, accel_divergence<NBX>(P, p, 1.0f / r0, src));
 }
 
 template <int NBX>
@@ -3199,11 +3238,9 @@ __global__ void __launch_bounds__(32 * CHECK_WARPS) k_sums2_warps(DevP P, int wi
 // ---------------------------------------------------------------------------------------- apply pressure
 // pressure.py:393-414 (lone particles: a push limited like a rigid contact's depenetration) and 461-480
 // (v += dt a, warm start stored dt-free). A lone particle has no neighbours, so no other particle reads its kappa.
-template <int NBX>
-__global__ void __launch_bounds__(BLOCK) k_apply(DevP P) {
-  constexpr bool MS = (NBX & MS_FLAG) != 0;
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.nfw[0]) return;
+// `accel(ax, ay, az)`: the pressure acceleration of p, from kappa and kr as they stand after the lone particle's limit.
+template <bool MS, class A>
+__device__ __forceinline__ void apply_with(const DevP& P, int p, A accel) {
   const float dt = P.dt;
   float4 vi = P.vel[p];
   float kap = P.kappa[p];
@@ -3242,7 +3279,7 @@ __global__ void __launch_bounds__(BLOCK) k_apply(DevP P) {
     }
   }
   float ax, ay, az;
-  pressure_accel<NBX>(P, p, P.pos[p], ax, ay, az);
+  accel(ax, ay, az);
   P.acc[p] = make_float4(ax, ay, az, 0.0f);
   float vx = ADF_FMA(dt, ax, vi.x), vy = ADF_FMA(dt, ay, vi.y), vz = ADF_FMA(dt, az, vi.z);
   // pressure.py:417-458: Coulomb friction of a lone particle on its walls after the update: the walls' push
@@ -3269,6 +3306,18 @@ __global__ void __launch_bounds__(BLOCK) k_apply(DevP P) {
   P.vel[p] = make_float4(vx, vy, vz, vi.w);
   if (P.mode == 0) P.kv_s[p] = kap * dt;
   else P.kd_s[p] = (kap * dt) * dt;
+}
+
+template <int NBX>
+__device__ __forceinline__ void apply_one(const DevP& P, int p) {
+  apply_with<(NBX & MS_FLAG) != 0>(
+      P, p, [&](float& ax, float& ay, float& az) { pressure_accel<NBX>(P, p, P.pos[p], ax, ay, az); });
+}
+
+template <int NBX>
+__global__ void __launch_bounds__(BLOCK) k_apply(DevP P) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < P.nfw[0]) apply_one<NBX>(P, p);
 }
 
 // ----------------------------------------------------------------------------------------- non-pressure
