@@ -12,9 +12,10 @@
 #include <vector>
 
 #include "../../include/alloy_dfsph.h"
+#include "dfsph_group.cuh"
+#include "dfsph_small.cuh"
 #include "dfsph_kernels.cuh"
 #include "dfsph_mlp.cuh"
-#include "dfsph_persist.cuh"
 #include "dfsph_port.cuh"
 #include "dfsph_skin.cuh"
 
@@ -193,15 +194,21 @@ struct adf_solver {
   bool warm_on = false, feat_rec = false, warm_alloc = false, judge = true;
   bool cg = false;  // projected preconditioned CG pressure solve (adf_params.cg)
   bool cg_team = false;  // CG products by teams of TL lanes per particle (models of at most CG_TEAM_MAX particles)
-  // the persistent CG solve (k_cg_solve) of team-product models, when adf_set_persistent turned it on
-  bool persist_on = false;
+  // whole solves as one cooperative launch (dfsph_group.cuh)
+  int persist = -1;          // adf_set_persistent: 1, 0, or -1 (never called): grid_solves
+  int grid_blocks = 0;       // blocks of the launch (0: none)
+  int grid_threads = 0;      // threads of each
+  int least_priority = 0;
+  int grid_form = 0;         // 0 rows in shared memory (dfsph_small.cuh), 1 deep blocks, 2 wide (dfsph_group.cuh)
+  int solve_runs = 0;                     // capacity of a list of runs
+  int* solve_ctr = nullptr;  // [2][CT_SIZE], one set per solve of a step (zeroed with the sort)
+  int2* solve_items = nullptr;                          // [2][solve_runs]
+  int *solve_chunks = nullptr, *solve_worlds = nullptr;  // [2][n_chunks], [2][W]
   // item halos of the pressure iterations (adf_set_halo): -1 the tuner times both forms, 0 off (the default), 1 always
   int halo_mode = 0;
   int halo_items = 0;  // item numbers k_halo covers: n / 256 + W + 1
-  int persist_cap[2] = {0, 0};       // co-resident blocks of k_cg_solve<false/true> on this device
   unsigned persist_extra = 0;        // extra arrivals a barrier waits for (only the wait-expiry test sets it)
-  long long persist_wait = 1 << 22;  // polls of one barrier wait (about a second) before it gives up
-  unsigned* parrive = nullptr;       // device [1]: barrier arrivals of the running launch
+  long long persist_wait = 1 << 25;  // polls of one barrier wait (some twenty seconds) before it gives up
   int* perr = nullptr;               // device [1]: a barrier wait gave up
   // the resting-jitter rule (adf_params.jitter_speed > 0): per-world tolerance factor and its float64 sums
   float* jit_scale = nullptr;                 // [W]
@@ -575,52 +582,112 @@ void cg_iteration(adf_solver* s, DevP& P, cudaStream_t st) {
   LAUNCH(s, k_cg_direction, blocks(n), BLOCK, st, P);
 }
 
-// The CG solve as one persistent launch (k_cg_solve) for team-product models with chunks, outside profiled runs
-// (those time each kernel group of the multi-launch path).
-bool persistent_solve(const adf_solver* s, const DevP& P) {
-  return s->cg && s->cg_team && s->persist_on && !s->prof_on && P.n_chunks > 0 && s->W > 0;
+// Whether this solve runs as one cooperative launch (dfsph_group.cuh). Steps that time kernels (tuning, profiling) and
+// staged item halos take the kernels one by one, and so does a solver told to (adf_set_persistent 0). The launch was
+// the faster one at every size measured, or equal (four steps, one kernel per phase against one launch): 2,016
+// particles 1.26 against 0.84 ms, the 30k column 4.08 against 2.56, 123k 1.89 against 1.55, 250k 3.07 against 2.70, the
+// 1M dam break 9.30 against 8.76, 256 columns 24.1 against 20.9, 6 worlds 1.90 against 1.61, 160 worlds 17.6 against
+// 17.4, the pour's first 1,024 worlds 60.6 against 59.8.
+bool grid_solves(const adf_solver* s, const DevP& P) {
+  if (P.n_chunks == 0 || s->W == 0 || s->prof_on || s->grid_blocks == 0) return false;
+  if (s->persist == 1 && s->cg) return true;
+  return s->persist != 0 && !s->tuning && s->halo_mode == 0;
 }
 
-int persistent_cg(adf_solver* s, DevP& P, cudaStream_t st) {
-  const bool ms = s->d.slot_cap > 1;
-  int& cap = s->persist_cap[ms ? 1 : 0];
-  if (cap == 0) {
-    int per_sm = 0, sms = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ms ? k_cg_solve<true> : k_cg_solve<false>, BLOCK, 0));
-    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
-    cap = per_sm * sms;
-    if (cap <= 0) return fail(ADF_ERR_CUDA, "k_cg_solve: no block of it fits on an SM");
+// The launch's kernel for this model (slot layout, solver, one world or several) and form.
+const void* grid_kernel(const adf_solver* s) {
+  static const void* const table[] = {
+      (const void*)k_small_solve<false, false, false>, (const void*)k_small_solve<false, false, true>,
+      (const void*)k_small_solve<false, true, false>, (const void*)k_small_solve<false, true, true>,
+      (const void*)k_small_solve<true, false, false>, (const void*)k_small_solve<true, false, true>,
+      (const void*)k_small_solve<true, true, false>, (const void*)k_small_solve<true, true, true>,
+      (const void*)k_grid_solve<false, false, false, false>, (const void*)k_grid_solve<false, false, true, false>,
+      (const void*)k_grid_solve<false, true, false, false>, (const void*)k_grid_solve<false, true, true, false>,
+      (const void*)k_grid_solve<true, false, false, false>, (const void*)k_grid_solve<true, false, true, false>,
+      (const void*)k_grid_solve<true, true, false, false>, (const void*)k_grid_solve<true, true, true, false>,
+      (const void*)k_grid_solve<false, false, false, true>, (const void*)k_grid_solve<false, false, true, true>,
+      (const void*)k_grid_solve<false, true, false, true>, (const void*)k_grid_solve<false, true, true, true>,
+      (const void*)k_grid_solve<true, false, false, true>, (const void*)k_grid_solve<true, false, true, true>,
+      (const void*)k_grid_solve<true, true, false, true>, (const void*)k_grid_solve<true, true, true, true>,
+  };
+  return table[s->grid_form * 8 + (s->d.slot_cap > 1 ? 4 : 0) + (s->cg ? 2 : 0) + (s->W == 1 ? 1 : 0)];
+}
+
+// One solve (or, with init 0, its iterations and apply) in one launch.
+int grid_solve(adf_solver* s, const DevP& P, int mode, int init, cudaStream_t st) {
+  SolveArgs A{};
+  A.init = init;
+  A.ctr = s->solve_ctr + mode * CT_SIZE;
+  for (int k = 0; k < 2; ++k) {
+    A.items[k] = s->solve_items + (size_t)k * s->solve_runs;
+    A.chunks[k] = s->solve_chunks + (size_t)k * P.n_chunks;
+    A.worlds[k] = s->solve_worlds + (size_t)k * s->W;
   }
-  const int n = s->n;
-  CgPersist R{};
-  R.pt_blocks = blocks(n);
-  R.team_blocks = blocks((long long)n * TL);
-  R.warp_fold = s->max_world_chunks <= WARP_FOLD_MAX_CHUNKS ? 1 : 0;
-  R.sum_blocks = R.warp_fold ? (P.n_chunks + CHECK_WARPS - 1) / CHECK_WARPS : P.n_chunks;
-  R.w_blocks = blocks(s->W);
-  R.cap = P.max_it + 2;  // as the WHILE node's cap
-  const int grid = std::min(cap, std::max(std::max(R.pt_blocks, R.team_blocks), std::max(R.sum_blocks, R.w_blocks)));
-  R.expect = (unsigned)grid + s->persist_extra;
-  R.wait_limit = s->persist_wait;
-  R.arrive = s->parrive;
-  R.status = s->perr;
-  CK(cudaMemsetAsync(s->parrive, 0, sizeof(unsigned), st));
+  A.extra = s->persist_extra;
+  A.wait_limit = s->persist_wait;
+  A.status = s->perr;
+  A.iters_out = mode == 0 ? s->iters_div : s->iters_den;
+  A.mean_out = mode == 0 ? s->div_err : s->den_err;
+  A.max_out = mode == 0 ? nullptr : s->den_err_max;
+  CK(cudaMemsetAsync(A.ctr, 0, sizeof(int) * CT_SIZE, st));
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3(BLOCK);
-  cfg.dynamicSmemBytes = 0;
+  cfg.gridDim = dim3((unsigned)s->grid_blocks);
+  cfg.blockDim = dim3((unsigned)s->grid_threads);
+  cfg.dynamicSmemBytes = s->grid_form == 0 ? SMALL_SMEM : 0;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeCooperative;  // every block resident: the barriers wait on all of them
   at[0].val.cooperative = 1;
+  // one priority whatever the stream's: two solvers' launches on streams of different priorities would otherwise take
+  // SMs from each other with neither wholly resident; of equal ones the first is dispatched whole
+  at[1].id = cudaLaunchAttributePriority;
+  at[1].val.priority = s->least_priority;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
-  prof_begin(s, 5, st);
-  if (ms) CK(cudaLaunchKernelEx(&cfg, k_cg_solve<true>, P, R));
-  else CK(cudaLaunchKernelEx(&cfg, k_cg_solve<false>, P, R));
+  cfg.numAttrs = 2;
+  void* args[] = {const_cast<DevP*>(&P), &A};
+  CK(cudaLaunchKernelExC(&cfg, grid_kernel(s), args));
   ++s->launches;
-  prof_end(s, st);
-  return check_launch();
+  return ADF_OK;
+}
+
+// Shape of the cooperative launch, from the particles that are or can become liquid (`sph`). Up to SMALL_BLOCK of them
+// per SM their rows fit the SMs' shared memory (dfsph_small.cuh). Above, a thread each while the device holds that many:
+// every SM gets an even share. Above that, the form that takes fewer rounds (dfsph_group.cuh).
+int setup_grid_solve(adf_solver* s, int sph) {
+  const long long runs = (long long)s->n / RUN + s->W;
+  if (s->W == 0 || s->n == 0 || s->W > LIST_MAX_WORLDS || runs > LIST_MAX_ITEMS || s->d.n_chunks > LIST_MAX_ITEMS)
+    return ADF_OK;
+  int sms = 0;
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
+  int greatest = 0;
+  CK(cudaDeviceGetStreamPriorityRange(&s->least_priority, &greatest));
+  const long long deep = (long long)sms * GRID_BLOCK, wide = 2ll * sms * WIDE_BLOCK, n = std::max(sph, 1);
+  if (n <= (long long)sms * SMALL_BLOCK) {
+    s->grid_form = 0;
+    s->grid_threads = SMALL_BLOCK;
+    s->grid_blocks = std::min(sms, blocks(n, RUN));  // a barrier costs by its arrivals
+  } else if (100 * ((n + deep - 1) / deep) <= 118 * ((n + wide - 1) / wide)) {
+    s->grid_form = 1;
+    s->grid_threads = std::min(blocks(blocks(n, sms), RUN) * RUN, GRID_BLOCK);
+    s->grid_blocks = sms;
+  } else {
+    s->grid_form = 2;
+    s->grid_threads = WIDE_BLOCK;
+    s->grid_blocks = 2 * sms;
+  }
+  s->solve_runs = (int)runs;
+  const void* kernel = grid_kernel(s);
+  const size_t smem = s->grid_form == 0 ? SMALL_SMEM : 0;
+  if (smem) CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int per_sm = 0;
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, s->grid_threads, smem));
+  if ((long long)per_sm * sms < s->grid_blocks) {  // not all resident: one kernel per phase
+    s->grid_blocks = 0;
+    return ADF_OK;
+  }
+  int rc = s->alloc(&s->solve_ctr, 2 * CT_SIZE) | s->alloc(&s->solve_items, 2 * (size_t)runs) |
+           s->alloc(&s->solve_chunks, 2 * (size_t)std::max(s->d.n_chunks, 1)) | s->alloc(&s->solve_worlds, 2 * (size_t)s->W);
+  return rc ? ADF_ERR_CUDA : ADF_OK;
 }
 
 // The stop test of an iteration and the next iteration's work list (one launch: k_check_warps or k_check_fused).
@@ -741,9 +808,13 @@ int solve(adf_solver* s, DevP& P, int mode, double dt, cudaStream_t st, bool gra
   const int n = s->n, W = s->W;
   const bool first = mode == 0 || !s->prm.divergence_solve;  // the step's first solve records the features
   const bool warm = s->warm_on && W > 0;
-  CK(cudaMemsetAsync(P.err_orig, 0, sizeof(float) * n, st));
-  if (warm) CK(cudaMemsetAsync(P.err2, 0, sizeof(float) * n, st));
-  CK(cudaMemsetAsync(P.n_unconv, 0, sizeof(int), st));
+  const bool grid = grid_solves(s, P);
+  const bool whole = grid && !warm && !(first && s->feat_rec);  // the start too is the group launch's
+  if (!whole) {
+    CK(cudaMemsetAsync(P.err_orig, 0, sizeof(float) * n, st));
+    if (warm) CK(cudaMemsetAsync(P.err2, 0, sizeof(float) * n, st));
+    CK(cudaMemsetAsync(P.n_unconv, 0, sizeof(int), st));
+  }
   P.feat_on = (first && (s->warm_on || s->feat_rec)) ? 1 : 0;
   // under the judge only the worlds that evaluate the learned start in this step need features and predictions
   const bool subset = warm && first && s->judge && !s->cg && !s->feat_rec;
@@ -761,6 +832,7 @@ int solve(adf_solver* s, DevP& P, int mode, double dt, cudaStream_t st, bool gra
            p.jitter_ratio > 0.0 ? (const double*)s->jit_flow : nullptr, (float)dt, (float)p.jitter_speed,
            (float)p.jitter_ratio, (float)p.tol_den, (float)p.tol_den_min, s->jit_scale, s->den_tol);
   }
+  if (whole) return grid_solve(s, P, mode, 1, st);
   prof_begin(s, 4, st);
   run_tk(s, TK_SOLVE_INIT, st, P);
   prof_end(s, st);
@@ -791,14 +863,10 @@ int solve(adf_solver* s, DevP& P, int mode, double dt, cudaStream_t st, bool gra
   if (rc) return rc;
   const bool dual = warm && s->judge && !s->cg;  // the first-sweep judge is a Jacobi sweep
   if (dual) dual_iteration(s, P, st);
-  if (persistent_solve(s, P)) {  // the CG start and its iterations in one launch
-    rc = persistent_cg(s, P, st);
-    if (rc) return rc;
-  } else {
-    if (s->cg && W > 0) cg_init(s, P, st);
-    rc = graph ? capture_iterations(s, P, st) : host_iterations(s, P, st, dual ? 1 : 0);
-    if (rc) return rc;
-  }
+  if (grid) return grid_solve(s, P, mode, 0, st);
+  if (s->cg && W > 0) cg_init(s, P, st);
+  rc = graph ? capture_iterations(s, P, st) : host_iterations(s, P, st, dual ? 1 : 0);
+  if (rc) return rc;
   prof_begin(s, 8, st);
   {
     const TuneCfg& c = s->tune[TK_ACCEL];
@@ -1109,8 +1177,8 @@ int adf_create(const adf_params* params, const adf_model* m, int device, adf_sol
     rc |= s->alloc(&d.cg_sums, W);
     rc |= s->alloc(&d.cg_restart, W);
     rc |= s->alloc(&d.cg_act_new, W);
-    rc |= s->alloc(&d.part2, std::max<size_t>(cb.size(), 1));
   }
+  rc |= s->alloc(&d.part2, std::max<size_t>(cb.size(), 1));
   rc |= s->alloc(&d.converged, W);
   rc |= s->alloc(&d.iters, W);
   rc |= s->alloc(&d.err_mean, W);
@@ -1229,6 +1297,8 @@ int adf_create(const adf_params* params, const adf_model* m, int device, adf_sol
     std::vector<int8_t> ph(s->n);
     if (s->n > 0) CKC(cudaMemcpy(ph.data(), m->phase, s->n, cudaMemcpyDeviceToHost));
     std::vector<int> stack0(n, 0), top0(W, 0);
+    int sph = 0;
+    for (int8_t v : ph) sph += (v >= 0 || v == PH_HELD) ? 1 : 0;
     for (int w = 0; w < s->W; ++w) {
       std::vector<int> ids;
       for (int i = s->ws_host[w]; i < s->ws_host[w + 1]; ++i)
@@ -1242,6 +1312,12 @@ int adf_create(const adf_params* params, const adf_model* m, int device, adf_sol
     CKC(cudaMemcpy(s->port_top, top0.data(), sizeof(int) * W, cudaMemcpyHostToDevice));
     for (int* a : {s->port_taken, s->port_granted, s->port_absorbed, s->port_emitted, s->port_retired})
       CKC(cudaMemset(a, 0, sizeof(int) * W));
+    const int rc_grid = setup_grid_solve(s, sph);
+    if (rc_grid) return fin(rc_grid);
+  }
+  if (s->cg) {  // the cooperative solves compare with what they find
+    CKC(cudaMemset(d.cg_restart, 0, sizeof(int) * W));
+    CKC(cudaMemset(d.cg_act_new, 0, sizeof(int) * W));
   }
   CKC(cudaMemset(d.counts, 0, sizeof(int) * std::max(s->n_keys, 1)));
   CKC(cudaMemset(d.nfw, 0, sizeof(int) * 2));
@@ -1295,7 +1371,6 @@ int adf_create(const adf_params* params, const adf_model* m, int device, adf_sol
   CKC(cudaStreamCreateWithFlags(&s->body_stream, cudaStreamNonBlocking));
   CKC(cudaMalloc(&s->body_runs, 2 * sizeof(unsigned long long)));
   CKC(cudaMemset(s->body_runs, 0, 2 * sizeof(unsigned long long)));
-  CKC(cudaMalloc(&s->parrive, sizeof(unsigned)));
   CKC(cudaMalloc(&s->perr, sizeof(int)));
   CKC(cudaMemset(s->perr, 0, sizeof(int)));
   CKC(cudaEventCreate(&s->tev[0]));
@@ -1329,7 +1404,6 @@ void adf_destroy(adf_solver* s) {
   if (s->pinned) cudaFreeHost(s->pinned);
   if (s->list_entries) cudaFree(s->list_entries);
   if (s->body_runs) cudaFree(s->body_runs);
-  if (s->parrive) cudaFree(s->parrive);
   if (s->perr) cudaFree(s->perr);
   for (auto& g : s->graphs) cudaGraphExecDestroy(g.exec);
   if (s->cap_stream) cudaStreamDestroy(s->cap_stream);
@@ -1764,8 +1838,9 @@ int adf_halo_stats(adf_solver* s, int32_t* in_use, int64_t* stats, void* stream)
 
 int adf_set_persistent(adf_solver* s, int enable) {
   if (!s) return fail(ADF_ERR_VALUE, "adf_set_persistent: null solver");
-  if (s->persist_on != (enable != 0)) ++s->table_version;
-  s->persist_on = enable != 0;
+  const int mode = enable != 0 ? 1 : 0;
+  if (s->persist != mode) ++s->table_version;
+  s->persist = mode;
   return ADF_OK;
 }
 

@@ -2401,9 +2401,8 @@ struct Team {
   unsigned mask;   // the team's lanes
 };
 
-// The team of this thread in block `vb` of BLOCK threads (a launch's own block, or a persistent kernel's virtual one).
-__device__ __forceinline__ Team team_at(int vb, int& p) {
-  const int g = vb * BLOCK + threadIdx.x;
+__device__ __forceinline__ Team team_of(int& p) {
+  const int g = blockIdx.x * BLOCK + threadIdx.x;
   p = g / TL;
   Team tm;
   tm.t = g % TL;
@@ -2411,8 +2410,6 @@ __device__ __forceinline__ Team team_at(int vb, int& p) {
   tm.mask = ((1u << TL) - 1u) << tm.t0;
   return tm;
 }
-
-__device__ __forceinline__ Team team_of(int& p) { return team_at(blockIdx.x, p); }
 
 __device__ __forceinline__ int2 row_entry(const DevP& P, int p, int k) { return __ldcs(P.nbrjf + p + (size_t)k * P.n); }
 
@@ -2499,12 +2496,11 @@ __device__ __forceinline__ float accel_divergence_team(const DevP& P, int p, flo
   return ar;
 }
 
-// k_cg_accel by teams (grid: TL threads per particle). The kernels below are bodies run for one block `vb` of BLOCK
-// threads, launched one block each by their __global__ wrappers or looped over by the persistent solve (k_cg_solve).
+// k_cg_accel by teams (grid: TL threads per particle).
 template <bool MS>
-__device__ __forceinline__ void cg_accel_team_at(const DevP& P, const float* vec, const float* vr, int gated, int vb) {
+__global__ void __launch_bounds__(BLOCK) k_cg_accel_team(DevP P, const float* vec, const float* vr, int gated) {
   int p;
-  const Team tm = team_at(vb, p);
+  const Team tm = team_of(p);
   if (p >= P.nfw[0] || cg_skip(P, P.world_s[p], gated)) return;
   DevP Q = P;
   Q.kappa = const_cast<float*>(vec);
@@ -2514,17 +2510,12 @@ __device__ __forceinline__ void cg_accel_team_at(const DevP& P, const float* vec
   if (tm.t == 0) P.acc[p] = make_float4(ax, ay, az, 0.0f);
 }
 
-template <bool MS>
-__global__ void __launch_bounds__(BLOCK) k_cg_accel_team(DevP P, const float* vec, const float* vr, int gated) {
-  cg_accel_team_at<MS>(P, vec, vr, gated, blockIdx.x);
-}
-
 // k_cg_apply by teams
 template <bool MS>
-__device__ __forceinline__ void cg_apply_team_at(const DevP& P, const float* vec, float* out, int gated, int bias,
-                                                 int accumulate, int vb) {
+__global__ void __launch_bounds__(BLOCK) k_cg_apply_team(DevP P, const float* vec, float* out, int gated, int bias,
+                                                         int accumulate) {
   int p;
-  const Team tm = team_at(vb, p);
+  const Team tm = team_of(p);
   if (p >= P.nfw[0] || cg_skip(P, P.world_s[p], gated)) return;
   const float inv_r0 = 1.0f / P.vel[p].w;
   const float ar = accel_divergence_team<MS>(P, p, inv_r0, tm);
@@ -2540,15 +2531,9 @@ __device__ __forceinline__ void cg_apply_team_at(const DevP& P, const float* vec
   out[p] = v;
 }
 
-template <bool MS>
-__global__ void __launch_bounds__(BLOCK) k_cg_apply_team(DevP P, const float* vec, float* out, int gated, int bias,
-                                                         int accumulate) {
-  cg_apply_team_at<MS>(P, vec, out, gated, bias, accumulate, blockIdx.x);
-}
-
 // krylov.py:104-133: active set, z = M^-1 r on F (r = -w), first direction p = z; pair.x = r.z
-__device__ __forceinline__ void cg_init_at(const DevP& P, int vb) {
-  const int p = vb * BLOCK + threadIdx.x;
+__global__ void __launch_bounds__(BLOCK) k_cg_init(DevP P) {
+  const int p = blockIdx.x * BLOCK + threadIdx.x;
   if (p >= P.nfw[0]) return;
   const float dt = P.dt;
   const float scale = P.mode == 0 ? dt : dt * dt;
@@ -2562,21 +2547,17 @@ __device__ __forceinline__ void cg_init_at(const DevP& P, int vb) {
   P.cg_pair[P.id_of[p]] = make_float2(-w * zi, 0.0f);
 }
 
-__global__ void __launch_bounds__(BLOCK) k_cg_init(DevP P) { cg_init_at(P, blockIdx.x); }
-
-__device__ __forceinline__ void cg_first_rz_at(const DevP& P, int vb) {
-  const int w = vb * BLOCK + threadIdx.x;
+__global__ void __launch_bounds__(BLOCK) k_cg_first_rz(DevP P) {
+  const int w = blockIdx.x * BLOCK + threadIdx.x;
   if (w >= P.W) return;
   P.cg_rz[w] = P.cg_sums[w].x;
   P.cg_restart[w] = 0;
   P.cg_act_new[w] = 0;
 }
 
-__global__ void __launch_bounds__(BLOCK) k_cg_first_rz(DevP P) { cg_first_rz_at(P, blockIdx.x); }
-
 // krylov.py:146-170: k += a p on F, projected onto k >= k_lo (the clamped part into corr); w += a A p
-__device__ __forceinline__ void cg_step_at(const DevP& P, int vb) {
-  const int p = vb * BLOCK + threadIdx.x;
+__global__ void __launch_bounds__(BLOCK) k_cg_step(DevP P) {
+  const int p = blockIdx.x * BLOCK + threadIdx.x;
   if (p >= P.nfw[0]) return;
   const int w = P.world_s[p];
   if (P.converged[w]) return;
@@ -2600,8 +2581,6 @@ __device__ __forceinline__ void cg_step_at(const DevP& P, int vb) {
   P.cg_corrr[p] = c / r0;
   P.cg_w[p] = ADF_FMA(a, P.cg_ap[p], P.cg_w[p]);
 }
-
-__global__ void __launch_bounds__(BLOCK) k_cg_step(DevP P) { cg_step_at(P, blockIdx.x); }
 
 // krylov.py:148-204 after the step: in worlds where k_cg_step clamped a variable, w += A corr (the correction
 // product of k_cg_apply: its acceleration field comes from k_cg_accel, launched for the same worlds); then in every
@@ -2650,9 +2629,9 @@ __global__ void __launch_bounds__(BLOCK) k_cg_apply_finish(DevP P) {
 
 // k_cg_apply_finish by teams
 template <bool MS>
-__device__ __forceinline__ void cg_apply_finish_team_at(const DevP& P, int vb) {
+__global__ void __launch_bounds__(BLOCK) k_cg_apply_finish_team(DevP P) {
   int p;
-  const Team tm = team_at(vb, p);
+  const Team tm = team_of(p);
   if (p >= P.nfw[0]) return;
   const int w = P.world_s[p];
   if (P.converged[w]) return;
@@ -2671,9 +2650,6 @@ __device__ __forceinline__ void cg_apply_finish_team_at(const DevP& P, int vb) {
   }
   if (tm.t == 0) cg_finish_one(P, p, w, wv, scale, div);
 }
-
-template <bool MS>
-__global__ void __launch_bounds__(BLOCK) k_cg_apply_finish_team(DevP P) { cg_apply_finish_team_at<MS>(P, blockIdx.x); }
 
 // krylov.py:207-233: per world the stop test (as k_world_check), then beta = r.z_new / r.z (0 after a set change)
 __device__ __forceinline__ void cg_beta_world(const DevP& P, int w) {
@@ -2700,8 +2676,8 @@ __global__ void k_cg_beta(DevP P) {
 }
 
 // krylov.py:236-246: p = z + beta p on F, 0 elsewhere
-__device__ __forceinline__ void cg_direction_at(const DevP& P, int vb) {
-  const int p = vb * BLOCK + threadIdx.x;
+__global__ void __launch_bounds__(BLOCK) k_cg_direction(DevP P) {
+  const int p = blockIdx.x * BLOCK + threadIdx.x;
   if (p >= P.nfw[0]) return;
   const int w = P.world_s[p];
   if (P.converged[w]) return;
@@ -2709,8 +2685,6 @@ __device__ __forceinline__ void cg_direction_at(const DevP& P, int vb) {
   P.cg_pd[p] = pd;
   P.cg_pdr[p] = pd / P.vel[p].w;
 }
-
-__global__ void __launch_bounds__(BLOCK) k_cg_direction(DevP P) { cg_direction_at(P, blockIdx.x); }
 
 // Per-world (sum x, sum y, max y) of the CG pairs for models without chunks (no particles): one block per world in
 // the fixed tree order of k_world_check; k_sums2_fused does it in one launch otherwise.
@@ -3063,12 +3037,12 @@ __global__ void __launch_bounds__(32 * CHECK_WARPS) k_check_warps(DevP P) {
 // The CG reductions in one launch (chunk partials and k_world_sum2's world fold, same tree order); with `beta`
 // the world's last block also runs k_cg_beta's stop test and beta for its world, and the grid's last block stores the
 // count of worlds still iterating as the unconverged count.
-__device__ __forceinline__ void sums2_fused_at(const DevP& P, int with_max, int beta, int vb) {
+__global__ void __launch_bounds__(256) k_sums2_fused(DevP P, int with_max, int beta) {
   __shared__ double smd[8];
   __shared__ float smf[8];
   __shared__ int smi[32];
   __shared__ bool wlast, glast;
-  const int c = vb;
+  const int c = blockIdx.x;
   const int w = P.chunk_world[c];
   const int c0 = P.world_chunk_start[w], c1 = P.world_chunk_start[w + 1];
   bool ticket = c == c0;  // as in k_check_fused
@@ -3119,10 +3093,6 @@ __device__ __forceinline__ void sums2_fused_at(const DevP& P, int with_max, int 
   }
 }
 
-__global__ void __launch_bounds__(256) k_sums2_fused(DevP P, int with_max, int beta) {
-  sums2_fused_at(P, with_max, beta, blockIdx.x);
-}
-
 // fold256_warp for two sums at once (value(L, x, y) gives value L of each)
 template <class F>
 __device__ __forceinline__ void fold256_warp2(F value, double& rx, double& ry) {
@@ -3152,12 +3122,12 @@ __device__ __forceinline__ void fold256_warp2(F value, double& rx, double& ry) {
 
 // k_sums2_fused with one warp per chunk (8 per block), for models whose worlds have at most WARP_FOLD_MAX_CHUNKS
 // chunks: the same partials, world folds, stop tests, beta and unconverged count in the same tree orders.
-__device__ __forceinline__ void sums2_warps_at(const DevP& P, int with_max, int beta, int vb) {
+__global__ void __launch_bounds__(32 * CHECK_WARPS) k_sums2_warps(DevP P, int with_max, int beta) {
   __shared__ int tickets[CHECK_WARPS];
   __shared__ int smi[32];
   __shared__ bool glast;
   const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
-  const int c = vb * CHECK_WARPS + wq;
+  const int c = blockIdx.x * CHECK_WARPS + wq;
   int ticket = 0;
   if (c < P.n_chunks) {
     const int w = P.chunk_world[c];
@@ -3229,10 +3199,6 @@ __device__ __forceinline__ void sums2_warps_at(const DevP& P, int with_max, int 
     block_exclusive_scan(open, smi, tot);
     if (threadIdx.x == 0) *P.n_unconv = tot;
   }
-}
-
-__global__ void __launch_bounds__(32 * CHECK_WARPS) k_sums2_warps(DevP P, int with_max, int beta) {
-  sums2_warps_at(P, with_max, beta, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------------------- apply pressure

@@ -432,9 +432,9 @@ class SolverDFSPH:
         _lib.check(self._lib.adf_set_autotune(self._h, int(bool(enable))), "autotune")
 
     def persistent(self, enable: bool = True) -> None:
-        """Run each projected-CG pressure solve of a model of at most 131,072 particles as one persistent launch with
-        grid-wide barriers (include/alloy_dfsph.h adf_set_persistent; off by default, the multi-launch path measured
-        slightly faster). The results are the same bits either way."""
+        """Whole pressure solves as one cooperative launch with grid-wide barriers (include/alloy_dfsph.h
+        adf_set_persistent), which a new solver does by itself; False: one kernel per phase. The results are the same
+        bits either way."""
         _lib.check(self._lib.adf_set_persistent(self._h, int(bool(enable))), "persistent")
 
     def halo(self, mode: int = 1) -> None:

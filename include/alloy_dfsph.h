@@ -179,20 +179,22 @@ int adf_set_halo(adf_solver* solver, int mode);
  * records. Synchronises `stream`. */
 int adf_halo_stats(adf_solver* solver, int32_t* in_use, int64_t* stats, void* stream);
 
-/* Persistent CG solve (no reference counterpart; the reference launches each CG kernel per iteration, krylov.py:254-297,
- * inside wp.capture_while, solve_driver.py:186). With the projected CG on models of at most 131,072 particles, each
- * pressure solve (its start and every iteration) runs as ONE cooperative launch whose phases are separated by
- * grid-wide barriers, instead of about nine launches per iteration; the results are the multi-launch path's bit for
- * bit. enable = 1 uses it wherever it applies (not in steps timed kernel by kernel, which take the multi-launch path);
- * 0 (the default at creation) takes the multi-launch path, which measured 2-4 % faster on a B200: under a replayed
- * step graph a grid barrier costs about what a kernel boundary does. Every barrier wait is bounded: a wait that gives
- * up sets the solver's status, after which adf_get_report returns ADF_ERR_STATE until adf_clear_status. */
+/* Whole solves as one launch (no reference counterpart; the reference launches each kernel per iteration, krylov.py:
+ * 254-297, inside wp.capture_while, solve_driver.py:186). Each pressure solve, its start, every iteration of every world
+ * and the velocity update, runs as ONE cooperative launch whose phases are separated by grid-wide barriers, instead of
+ * four graph nodes per Jacobi iteration or ten per CG iteration; the results are the same bits. This is what a new
+ * solver does, except in steps that time kernels one by one (tuning, profiling) and with item halos on. enable = 1 does
+ * it in the tuning step too, for the projected CG; 0 launches one kernel per phase. Every barrier wait is bounded: a
+ * wait that gives up sets the solver's status, after which adf_get_report returns ADF_ERR_STATE until
+ * adf_clear_status. The launch occupies every SM of the device it finds free and is dispatched at the lowest stream
+ * priority. */
 int adf_set_persistent(adf_solver* solver, int enable);
-/* Test hook of the bounded barrier waits: each wait polls at most `polls` times (default 4,194,304, about a second),
+/* Test hook of the bounded barrier waits: each wait polls at most `polls` times (default 33,554,432, some twenty
+ * seconds),
  * and a barrier waits for `extra_arrivals` more blocks than the grid has (default 0; any other value makes every wait
  * run out, which is what the wait-expiry test checks). */
 int adf_set_barrier_wait(adf_solver* solver, long long polls, int extra_arrivals);
-/* Clears the status words of the bounded waits (the persistent solve's barriers and the warm-start network's
+/* Clears the status words of the bounded waits (the solves' grid barriers and the warm-start network's
  * tensor-core waits) and the per-world reduction tickets a launch that gave up may have left counted, after
  * synchronising the device. */
 int adf_clear_status(adf_solver* solver);
