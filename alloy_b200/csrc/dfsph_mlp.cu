@@ -45,8 +45,8 @@ int set_params(adf_mlp* m, const float* host) {
 int grad_launch(adf_mlp* m, const float* x, const float* y, const int32_t* idx, int batch, cudaStream_t st,
                 int* grid_out) {
   const int tiles = (batch + TILE - 1) / TILE;
-  const int grid = std::max(1, std::min(tiles, m->sms));
-  k_mlp_grad<<<grid, TILE, TR_SMEM, st>>>(net_of(m), x, y, idx, batch, m->part);
+  const int grid = std::max(1, std::min(tiles, TR_CTAS * m->sms));
+  k_mlp_grad<<<grid, TR_THREADS, TR_SMEM, st>>>(net_of(m), x, y, idx, batch, m->part);
   CKM(cudaGetLastError());
   *grid_out = grid;
   return ADF_OK;
@@ -73,7 +73,7 @@ int adf_mlp_create(const float* params, int device, adf_mlp** out) {
   al((void**)&m->v, sizeof(float) * N_PARAMS);
   al((void**)&m->w1b, sizeof(__nv_bfloat16) * NH * NF);
   al((void**)&m->w2b, sizeof(__nv_bfloat16) * NH * NH);
-  al((void**)&m->part, sizeof(float) * (size_t)m->sms * (N_PARAMS + 1));
+  al((void**)&m->part, sizeof(float) * (size_t)TR_CTAS * m->sms * (N_PARAMS + 1));
   al((void**)&m->grad, sizeof(float) * N_PARAMS);
   al((void**)&m->loss, sizeof(float));
   al((void**)&m->error, sizeof(int));
@@ -136,7 +136,7 @@ int adf_mlp_gradient(adf_mlp* m, const float* x, const float* y, const int32_t* 
   int grid = 0;
   int rc = grad_launch(m, x, y, idx, batch, st, &grid);
   if (rc) return rc;
-  k_mlp_adam<<<(N_PARAMS + 256) / 256, 256, 0, st>>>(m->part, grid, batch, m->w, m->m, m->v, m->w1b, m->w2b, 0.0f,
+  k_mlp_adam<<<N_PARAMS / ADAM_PARAMS + 1, ADAM_PARAMS * ADAM_SPLIT, 0, st>>>(m->part, grid, batch, m->w, m->m, m->v, m->w1b, m->w2b, 0.0f,
                                                       0.9f, 0.999f, 1e-8f, 1, 0, m->grad, m->loss);
   CKM(cudaGetLastError());
   CKM(cudaStreamSynchronize(st));
@@ -155,7 +155,7 @@ int adf_mlp_train_step(adf_mlp* m, const float* x, const float* y, const int32_t
   int rc = grad_launch(m, x, y, idx, batch, st, &grid);
   if (rc) return rc;
   ++m->step;
-  k_mlp_adam<<<(N_PARAMS + 256) / 256, 256, 0, st>>>(m->part, grid, batch, m->w, m->m, m->v, m->w1b, m->w2b, lr,
+  k_mlp_adam<<<N_PARAMS / ADAM_PARAMS + 1, ADAM_PARAMS * ADAM_SPLIT, 0, st>>>(m->part, grid, batch, m->w, m->m, m->v, m->w1b, m->w2b, lr,
                                                       0.9f, 0.999f, 1e-8f, m->step, 1, nullptr, m->loss);
   CKM(cudaGetLastError());
   if (loss) {

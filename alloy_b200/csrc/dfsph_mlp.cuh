@@ -376,16 +376,31 @@ constexpr int TR_H = TR_X + TILE * NF * 2;            // A of layer 2: 128 x 64
 constexpr int TR_DZ2 = TR_H + TILE * NH * 2;          // A of dH1: 128 x 64
 constexpr int TR_AWG = TR_DZ2 + TILE * NH * 2;        // A of the weight gradients: 128 x 128 ([dZ2^T ; dZ1^T])
 constexpr int TR_BWG = TR_AWG + TILE * TILE * 2;      // B of the weight gradients: 96 x 128 ([H1 | X | 1 | 0]^T)
-constexpr int TR_F = TR_BWG + N_WG * TILE * 2;        // FP32: b1 64, b2 64, w3 128, b3 2, acc w3 128, acc b3 2, loss
-constexpr int TR_BAR = TR_F + (64 + 64 + 128 + 4 + 128 + 4) * 4;
-constexpr int TR_SMEM = TR_BAR + 16;  // ~112 KB: at most 2 CTAs per SM, 2 x 256 TMEM columns
+constexpr int TR_F = TR_BWG + N_WG * TILE * 2;        // FP32: b1 64, b2 64, w3 128, b3 2 (+ 2 pad), dy 128 x 2
+constexpr int TR_BAR = TR_F + (64 + 64 + 128 + 4 + 2 * TILE) * 4;
+constexpr int TR_SMEM = TR_BAR + 16;  // ~112 KB: 2 CTAs per SM, 2 x 256 TMEM columns
 constexpr int TR_TMEM_COLS = 256;     // [0, 64) Z1, [64, 128) Z2 then dH1, [128, 224) weight gradients
 constexpr int TR_C_WG = 128;
+constexpr int TR_THREADS = 2 * TILE;  // two threads per row, each half of its 64 columns
+constexpr int TR_CTAS = 2;            // CTAs per SM
+// h2 of the rows, 32 columns at a time, for the output layer's gradient: FP32 over X and H, which the tile's first two
+// MMAs have read by then.
+constexpr int TR_HB = TR_X, TR_HB_LD = 33;
+static_assert(TILE * TR_HB_LD * 4 <= TR_DZ2 - TR_HB, "the h2 columns fit over X and H");
+static_assert(TR_CTAS * (TR_SMEM + 1024) <= 228 * 1024, "two CTAs' shared memory fits an SM");
 
 // Per-CTA gradient of the mean squared error over the batch (rows idx[0 .. batch)), written to part[cta][N_PARAMS + 1]
 // (the last element: the CTA's summed squared error). x: [N][16] normalised features, y: [N][2] normalised targets.
-__global__ void __launch_bounds__(TILE) k_mlp_grad(Net net, const float* __restrict__ x, const float* __restrict__ y,
-                                                   const int* __restrict__ idx, int batch, float* part) {
+//
+// A tile is a chain (four MMAs of a microsecond each between epilogues that every row's thread runs), so what counts is
+// the threads that share the epilogues and the tiles an SM has in flight: two threads a row and two CTAs an SM, against
+// one and one before, where four warps held an SM. The output layer's gradient dW3 = sum over rows of dy h2 is kept in
+// registers: the tile's h2 passes through shared memory 32 columns at a time and each thread sums 32 rows of one (output,
+// column), against ten shuffles and two shared atomics for each of the 64 columns before. A training step of 65,536 rows
+// went from 120 to 48 us, Adam included.
+__global__ void __launch_bounds__(TR_THREADS, TR_CTAS) k_mlp_grad(Net net, const float* __restrict__ x,
+                                                                  const float* __restrict__ y,
+                                                                  const int* __restrict__ idx, int batch, float* part) {
   extern __shared__ __align__(128) unsigned char smem[];
   unsigned char* sW1 = smem + TR_W1;
   unsigned char* sW2 = smem + TR_W2;
@@ -400,33 +415,33 @@ __global__ void __launch_bounds__(TILE) k_mlp_grad(Net net, const float* __restr
   float* b2 = sF + 64;
   float* w3 = sF + 128;
   float* b3 = sF + 256;
-  float* gw3 = sF + 260;
-  float* gb3 = sF + 388;   // [2], then the summed squared error at [2]
+  float2* sdy = reinterpret_cast<float2*>(sF + 260);  // [TILE]
+  float* hb = reinterpret_cast<float*>(smem + TR_HB);  // [TILE][TR_HB_LD]
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + TR_BAR);
   __shared__ uint32_t tmem_base;
-  const int t = threadIdx.x;
-  const int lane = t & 31;
+  const int t = threadIdx.x % TILE, half = threadIdx.x / TILE;
+  const int lane = threadIdx.x & 31;
+  const int col0 = 32 * half;  // this thread's columns of the hidden layers
+  // this thread's share of dW3: output og of column cg of the staged 32, rows [32 rg, 32 rg + 32)
+  const int cg = threadIdx.x & 31, og = (threadIdx.x >> 5) & 1, rg = threadIdx.x >> 6;
+  float gw3[2] = {0.0f, 0.0f};
 
   load_operand(sW1, net.w1, NH, NF);
   load_operand(sW2, net.w2, NH, NH);
   load_operand_t(sW2T, net.w2, NH, NH);
-  for (int e = t; e < 64; e += blockDim.x) {
+  for (int e = threadIdx.x; e < 64; e += blockDim.x) {
     b1[e] = net.p[OFF_B1 + e];
     b2[e] = net.p[OFF_B2 + e];
   }
-  for (int e = t; e < 128; e += blockDim.x) {
-    w3[e] = net.p[OFF_W3 + e];
-    gw3[e] = 0.0f;
-  }
-  if (t < 2) b3[t] = net.p[OFF_B3 + t];
-  if (t < 4) gb3[t] = 0.0f;
+  for (int e = threadIdx.x; e < 128; e += blockDim.x) w3[e] = net.p[OFF_W3 + e];
+  if (threadIdx.x < 2) b3[threadIdx.x] = net.p[OFF_B3 + threadIdx.x];
   // constant columns of B_wg: row 80 = ones, rows 81..95 = zero (rows of B are its N index)
-  for (int e = t; e < 16 * TILE; e += blockDim.x) {
+  for (int e = threadIdx.x; e < 16 * TILE; e += blockDim.x) {
     const int n = 80 + e / TILE, k = e % TILE;
     st_bf16(sBwg, kmaj(n, k, TILE), n == 80 ? 1.0f : 0.0f);
   }
-  if (t == 0) mbar_init(bar, 1);
-  if (t < 32) {
+  if (threadIdx.x == 0) mbar_init(bar, 1);
+  if (threadIdx.x < 32) {
     tmem_alloc(&tmem_base, TR_TMEM_COLS);
     tmem_relinquish();
   }
@@ -445,7 +460,8 @@ __global__ void __launch_bounds__(TILE) k_mlp_grad(Net net, const float* __restr
   int done = 0;  // tiles whose weight gradients are in TMEM
   const float inv_b = 1.0f / (float)max(batch, 1);
   const int tiles = (batch + TILE - 1) / TILE;
-  float sq = 0.0f;
+  float sq = 0.0f, gb0 = 0.0f, gb1 = 0.0f;  // of this thread's rows (half 0)
+  const bool wide = (reinterpret_cast<uintptr_t>(x) & 15) == 0;  // rows on 16-byte boundaries
   auto wait = [&]() -> bool {
     ++committed;
     failed = !mbar_wait(bar, phase, net.wait_limit);
@@ -465,102 +481,110 @@ __global__ void __launch_bounds__(TILE) k_mlp_grad(Net net, const float* __restr
     const int r = tile * TILE + t;
     const bool valid = r < batch;
     const int s = valid ? idx[r] : 0;
-    float xr[NF], tg0 = 0.0f, tg1 = 0.0f;
+    float2 tg = make_float2(0.0f, 0.0f);
+    {  // each thread of a row takes half of its features
+      float xr[8];
+      const float* xs = x + (size_t)s * NF + 8 * half;
 #pragma unroll
-    for (int k = 0; k < NF; ++k) xr[k] = valid ? x[(size_t)s * NF + k] : 0.0f;
-    if (valid) {
-      tg0 = y[2 * (size_t)s];
-      tg1 = y[2 * (size_t)s + 1];
-    }
+      for (int q = 0; q < 2; ++q) {
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (valid && wide) v = *reinterpret_cast<const float4*>(xs + 4 * q);
+        else if (valid) v = make_float4(xs[4 * q], xs[4 * q + 1], xs[4 * q + 2], xs[4 * q + 3]);
+        xr[4 * q] = v.x;
+        xr[4 * q + 1] = v.y;
+        xr[4 * q + 2] = v.z;
+        xr[4 * q + 3] = v.w;
+      }
+      if (valid && half == 0) tg = make_float2(y[2 * (size_t)s], y[2 * (size_t)s + 1]);
+      st_row8(sX, kmaj(t, 8 * half, NF), xr);
 #pragma unroll
-    for (int k = 0; k < NF; ++k) {
-      st_bf16(sX, kmaj(t, k, NF), xr[k]);
-      st_bf16(sBwg, kmaj(64 + k, t, TILE), xr[k]);
+      for (int k = 0; k < 8; ++k) st_bf16(sBwg, kmaj(64 + 8 * half + k, t, TILE), xr[k]);
     }
     sync_for_mma();
-    if (t == 0) {
+    if (threadIdx.x == 0) {
       mma_bf16(tm, dX, dW1, id64, 0);
       mma_commit(bar);
     }
     if (!wait()) break;
     // layer 1 epilogue: H1 as the A operand of layer 2 and as rows 0..63 of B_wg
 #pragma unroll
-    for (int c = 0; c < NH; c += 16) {
+    for (int c = col0; c < col0 + 32; c += 16) {
       float v[16];
       tmem_ld16(tmem_row(tm, c), v);
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         const float z = v[i] + b1[c + i];
-        const float h = z * sigmoid(z);
-        st_bf16(sH, kmaj(t, c + i, NH), h);
-        st_bf16(sBwg, kmaj(c + i, t, TILE), h);
+        v[i] = z * sigmoid(z);
+        st_bf16(sBwg, kmaj(c + i, t, TILE), v[i]);
       }
+      st_row8(sH, kmaj(t, c, NH), v);
+      st_row8(sH, kmaj(t, c + 8, NH), v + 8);
     }
     sync_for_mma();
-    if (t == 0) {
+    if (threadIdx.x == 0) {
 #pragma unroll
       for (int k = 0; k < NH / 16; ++k)
         mma_bf16(tm + 64, dH + (uint64_t)(k * 16), dW2 + (uint64_t)(k * 16), id64, k > 0);
       mma_commit(bar);
     }
     if (!wait()) break;
-    // output and loss gradient (dL/dy = (y - t) / batch for L = sum (y - t)^2 / (2 batch))
-    float y0 = b3[0], y1 = b3[1];
+    // output and loss gradient (dL/dy = (y - t) / batch for L = sum (y - t)^2 / (2 batch)): each half's share of the
+    // outputs, the second half's through shared memory
+    float z2[32], s2[32];
+    float y0 = half == 0 ? b3[0] : 0.0f, y1 = half == 0 ? b3[1] : 0.0f;
 #pragma unroll
-    for (int c = 0; c < NH; c += 16) {
+    for (int c = 0; c < 32; c += 16) {
       float v[16];
-      tmem_ld16(tmem_row(tm, 64 + c), v);
+      tmem_ld16(tmem_row(tm, 64 + col0 + c), v);
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
-        const float z = v[i] + b2[c + i];
-        const float h = z * sigmoid(z);
-        y0 = fmaf(w3[c + i], h, y0);
-        y1 = fmaf(w3[64 + c + i], h, y1);
-      }
-    }
-    const float e0 = valid ? y0 - tg0 : 0.0f, e1 = valid ? y1 - tg1 : 0.0f;
-    sq = fmaf(e0, e0, fmaf(e1, e1, sq));
-    const float dy0 = e0 * inv_b, dy1 = e1 * inv_b;
-    // dZ2 = (W3^T dy) * silu'(z2); dW3 += dy h2^T (warp sums, then shared atomics)
-#pragma unroll
-    for (int c = 0; c < NH; c += 16) {
-      float v[16];
-      tmem_ld16(tmem_row(tm, 64 + c), v);
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const int j = c + i;
+        const int j = col0 + c + i;
         const float z = v[i] + b2[j];
         const float sg = sigmoid(z);
         const float h = z * sg;
-        const float dz = fmaf(w3[j], dy0, w3[64 + j] * dy1) * (sg * fmaf(z, 1.0f - sg, 1.0f));
-        st_bf16(sDZ2, kmaj(t, j, NH), dz);
-        st_bf16(sAwg, kmaj(j, t, TILE), dz);
-        float g0 = dy0 * h, g1 = dy1 * h;
-#pragma unroll
-        for (int o = 16; o >= 1; o >>= 1) {
-          g0 += __shfl_xor_sync(0xffffffffu, g0, o);
-          g1 += __shfl_xor_sync(0xffffffffu, g1, o);
-        }
-        if (lane == 0) {
-          atomicAdd(&gw3[j], g0);
-          atomicAdd(&gw3[64 + j], g1);
-        }
+        z2[c + i] = z;
+        s2[c + i] = sg;
+        y0 = fmaf(w3[j], h, y0);
+        y1 = fmaf(w3[64 + j], h, y1);
       }
     }
-    {
-      float g0 = dy0, g1 = dy1;
+    if (half == 1) sdy[t] = make_float2(y0, y1);
+    __syncthreads();
+    if (half == 0) {
+      const float2 o = sdy[t];
+      const float e0 = valid ? (y0 + o.x) - tg.x : 0.0f, e1 = valid ? (y1 + o.y) - tg.y : 0.0f;
+      sq = fmaf(e0, e0, fmaf(e1, e1, sq));
+      const float2 dy = make_float2(e0 * inv_b, e1 * inv_b);
+      gb0 += dy.x;
+      gb1 += dy.y;
+      sdy[t] = dy;
+    }
+    __syncthreads();
+    // dZ2 = (W3^T dy) * silu'(z2); dW3 += dy h2^T
+    const float2 dy = sdy[t];
 #pragma unroll
-      for (int o = 16; o >= 1; o >>= 1) {
-        g0 += __shfl_xor_sync(0xffffffffu, g0, o);
-        g1 += __shfl_xor_sync(0xffffffffu, g1, o);
+    for (int c = 0; c < 32; c += 16) {
+      float v[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const int j = col0 + c + i;
+        const float z = z2[c + i], sg = s2[c + i];
+        v[i] = fmaf(w3[j], dy.x, w3[64 + j] * dy.y) * (sg * fmaf(z, 1.0f - sg, 1.0f));
+        st_bf16(sAwg, kmaj(j, t, TILE), v[i]);
+        hb[t * TR_HB_LD + 16 * half + i] = z * sg;
       }
-      if (lane == 0) {
-        atomicAdd(&gb3[0], g0);
-        atomicAdd(&gb3[1], g1);
-      }
+      st_row8(sDZ2, kmaj(t, col0 + c, NH), v);
+      st_row8(sDZ2, kmaj(t, col0 + c + 8, NH), v + 8);
+      __syncthreads();
+      const float* dyo = reinterpret_cast<const float*>(sdy) + og;
+      float g = 0.0f;
+#pragma unroll 8
+      for (int k = 32 * rg; k < 32 * rg + 32; ++k) g = fmaf(dyo[2 * k], hb[k * TR_HB_LD + cg], g);
+      gw3[c / 16] += g;
+      if (c == 0) __syncthreads();
     }
     sync_for_mma();
-    if (t == 0) {  // dH1 = dZ2 W2 into the Z2 columns (Z2 is no longer needed)
+    if (threadIdx.x == 0) {  // dH1 = dZ2 W2 into the Z2 columns (Z2 is no longer needed)
 #pragma unroll
       for (int k = 0; k < NH / 16; ++k)
         mma_bf16(tm + 64, dDZ2 + (uint64_t)(k * 16), dW2T + (uint64_t)(k * 16), id64, k > 0);
@@ -569,7 +593,7 @@ __global__ void __launch_bounds__(TILE) k_mlp_grad(Net net, const float* __restr
     if (!wait()) break;
     // dZ1 = dH1 * silu'(z1) as rows 64..127 of A_wg
 #pragma unroll
-    for (int c = 0; c < NH; c += 16) {
+    for (int c = col0; c < col0 + 32; c += 16) {
       float dh[16], v[16];
       tmem_ld16(tmem_row(tm, 64 + c), dh);
       tmem_ld16(tmem_row(tm, c), v);
@@ -581,7 +605,7 @@ __global__ void __launch_bounds__(TILE) k_mlp_grad(Net net, const float* __restr
       }
     }
     sync_for_mma();
-    if (t == 0) {  // weight gradients, accumulated in TMEM over this CTA's tiles
+    if (threadIdx.x == 0) {  // weight gradients, accumulated in TMEM over this CTA's tiles
 #pragma unroll
       for (int k = 0; k < TILE / 16; ++k)
         mma_bf16(tm + TR_C_WG, dAwg + (uint64_t)(k * 16), dBwg + (uint64_t)(k * 16), idwg, (done > 0 || k > 0) ? 1u : 0u);
@@ -590,15 +614,8 @@ __global__ void __launch_bounds__(TILE) k_mlp_grad(Net net, const float* __restr
     if (!wait()) break;
     ++done;
   }
-  // the CTA's summed squared error
-  {
-    float g = sq;
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
-    if (lane == 0) atomicAdd(&gb3[2], g);
-  }
   if (failed) {
-    if (t == 0) atomicExch(net.error, 1);
+    if (threadIdx.x == 0) atomicExch(net.error, 1);
     for (int k = 0; k < committed; ++k) {
       mbar_wait(bar, phase, WAIT_LIMIT);
       phase ^= 1;
@@ -609,44 +626,81 @@ __global__ void __launch_bounds__(TILE) k_mlp_grad(Net net, const float* __restr
   tc_after();
   float* out = part + (size_t)blockIdx.x * (N_PARAMS + 1);
   const bool have = done > 0 && !failed;
-  if (t < 64) {  // rows 0..63: dW2 (cols 0..63) and db2 (col 80)
-    for (int c = 0; c < 96; c += 16) {
+  // the CTA's sums over rows, in a fixed order: dW3 over the four row groups, db3 and the squared error over the warps
+#pragma unroll
+  for (int c = 0; c < 2; ++c) hb[rg * 128 + og * 64 + (cg >> 4) * 32 + 16 * c + (cg & 15)] = gw3[c];
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) {
+    gb0 += __shfl_xor_sync(0xffffffffu, gb0, o);
+    gb1 += __shfl_xor_sync(0xffffffffu, gb1, o);
+    sq += __shfl_xor_sync(0xffffffffu, sq, o);
+  }
+  if (half == 0 && lane == 0) {
+    hb[512 + 3 * (t >> 5)] = gb0;
+    hb[513 + 3 * (t >> 5)] = gb1;
+    hb[514 + 3 * (t >> 5)] = sq;
+  }
+  __syncthreads();
+  if (threadIdx.x < 128) {
+    const int e = threadIdx.x;
+    out[OFF_W3 + e] = ((hb[e] + hb[128 + e]) + hb[256 + e]) + hb[384 + e];
+  } else if (threadIdx.x < 131) {
+    const int e = threadIdx.x - 128;
+    const float g = ((hb[512 + e] + hb[515 + e]) + hb[518 + e]) + hb[521 + e];
+    out[e < 2 ? OFF_B3 + e : N_PARAMS] = g;
+  }
+  if (t < 64) {  // rows 0..63: dW2 (cols 0..63, half of them each) and db2 (col 80)
+    for (int c = col0; c < col0 + 32; c += 16) {
       float v[16];
       tmem_ld16(tmem_row(tm, TR_C_WG + c), v);
-      if (c < 64) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) out[OFF_W2 + t * NH + c + i] = have ? v[i] : 0.0f;
-      } else if (c == 80) {
-        out[OFF_B2 + t] = have ? v[0] : 0.0f;
-      }
+      for (int i = 0; i < 16; ++i) out[OFF_W2 + t * NH + c + i] = have ? v[i] : 0.0f;
+    }
+    if (half == 0) {
+      float v[16];
+      tmem_ld16(tmem_row(tm, TR_C_WG + 80), v);
+      out[OFF_B2 + t] = have ? v[0] : 0.0f;
     }
   } else {  // rows 64..127: dW1 (cols 64..79) and db1 (col 80)
     const int m = t - 64;
     float v[16];
-    tmem_ld16(tmem_row(tm, TR_C_WG + 64), v);
+    tmem_ld16(tmem_row(tm, TR_C_WG + (half == 0 ? 64 : 80)), v);
+    if (half == 0) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) out[OFF_W1 + m * NF + i] = have ? v[i] : 0.0f;
-    tmem_ld16(tmem_row(tm, TR_C_WG + 80), v);
-    out[OFF_B1 + m] = have ? v[0] : 0.0f;
+      for (int i = 0; i < 16; ++i) out[OFF_W1 + m * NF + i] = have ? v[i] : 0.0f;
+    } else {
+      out[OFF_B1 + m] = have ? v[0] : 0.0f;
+    }
   }
-  for (int e = t; e < 128; e += blockDim.x) out[OFF_W3 + e] = gw3[e];
-  if (t < 2) out[OFF_B3 + t] = gb3[t];
-  if (t == 0) out[N_PARAMS] = gb3[2];
   tc_before();
   __syncthreads();
   tc_after();
-  if (t < 32) tmem_dealloc(tm, TR_TMEM_COLS);
+  if (threadIdx.x < 32) tmem_dealloc(tm, TR_TMEM_COLS);
 }
 
-// Sum of the CTA partials in CTA order (deterministic), then one Adam step on the FP32 master parameters and their
-// BF16 copies. grad_out (optional) receives the summed gradient; loss_out[0] the batch's mean squared error.
-__global__ void k_mlp_adam(const float* part, int n_part, int batch, float* w, float* m, float* v,
-                           __nv_bfloat16* w1b, __nv_bfloat16* w2b, float lr, float b1, float b2, float eps, int step,
-                           int apply, float* grad_out, float* loss_out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i > N_PARAMS) return;
+// Sum of the CTA partials in a fixed order (deterministic): eight threads a parameter, each every eighth partial, then
+// their sums in order; then one Adam step on the FP32 master parameters and their BF16 copies. grad_out (optional)
+// receives the summed gradient; loss_out[0] the batch's mean squared error. One thread a parameter, a chain of 148 loads
+// from few warps, took 10.5 us.
+constexpr int ADAM_PARAMS = 32, ADAM_SPLIT = 8;  // parameters of a block, threads a parameter
+
+__global__ void __launch_bounds__(ADAM_PARAMS * ADAM_SPLIT)
+k_mlp_adam(const float* part, int n_part, int batch, float* w, float* m, float* v, __nv_bfloat16* w1b,
+           __nv_bfloat16* w2b, float lr, float b1, float b2, float eps, int step, int apply, float* grad_out,
+           float* loss_out) {
+  __shared__ float sums[ADAM_SPLIT][ADAM_PARAMS];
+  const int lane = threadIdx.x % ADAM_PARAMS, q = threadIdx.x / ADAM_PARAMS;
+  const int i = blockIdx.x * ADAM_PARAMS + lane;
   float g = 0.0f;
-  for (int c = 0; c < n_part; ++c) g += part[(size_t)c * (N_PARAMS + 1) + i];
+  if (i <= N_PARAMS) {
+#pragma unroll 8
+    for (int c = q; c < n_part; c += ADAM_SPLIT) g += part[(size_t)c * (N_PARAMS + 1) + i];
+  }
+  sums[q][lane] = g;
+  __syncthreads();
+  if (q > 0 || i > N_PARAMS) return;
+#pragma unroll
+  for (int k = 1; k < ADAM_SPLIT; ++k) g += sums[k][lane];
   if (i == N_PARAMS) {
     if (loss_out) loss_out[0] = g / (float)(2 * max(batch, 1));
     return;
@@ -685,7 +739,7 @@ struct adf_mlp {
   float* v = nullptr;  // Adam second moments
   __nv_bfloat16* w1b = nullptr;
   __nv_bfloat16* w2b = nullptr;
-  float* part = nullptr;  // [sms][N_PARAMS + 1] per-CTA gradients
+  float* part = nullptr;  // [TR_CTAS sms][N_PARAMS + 1] per-CTA gradients
   float* grad = nullptr;  // [N_PARAMS]
   float* loss = nullptr;  // [1]
   int* error = nullptr;   // bounded-wait expiry flag
