@@ -8,6 +8,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -104,6 +105,9 @@ int fail(int code, const std::string& msg) {
     if (e_ != cudaSuccess) return -fail(ADF_ERR_CUDA, std::string(#x) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
+// Packed words of a report: three 8-byte and fifteen 4-byte arrays per world, two status words.
+inline size_t report_words(int W) { return (size_t)W * (3 * 2 + 15) + 2; }
+
 inline int blocks(long long n, int b = BLOCK) { return (int)((n + b - 1) / b); }
 
 // Models up to this many particles take the CG products by teams of TL lanes per particle: below it one lane per
@@ -164,6 +168,9 @@ struct adf_solver {
   int *cw2 = nullptr, *cseg2 = nullptr, *n_cw2 = nullptr;  // work list of the learned start's first sweep
   int* warm_need = nullptr;  // [W] worlds that evaluate the learned start in this step (k_warm_need)
   int* speed_bits = nullptr;
+  // the report's packed words (adf_get_report), and their pinned copy
+  int *report_dev = nullptr, *report_host = nullptr;
+  std::mutex report_mutex;
   // host side of the iteration loop
   int* pinned = nullptr;
   cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -1367,6 +1374,8 @@ int adf_create(const adf_params* params, const adf_model* m, int device, adf_sol
   CKC(cudaFuncSetAttribute(k_jacobi_h<16 | MS_FLAG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)HALO_SMEM_JACOBI));
   CKC(cudaHostAlloc((void**)&s->pinned, 2 * sizeof(int), cudaHostAllocDefault));
+  CKC(cudaMalloc(&s->report_dev, sizeof(int) * report_words(W)));
+  CKC(cudaHostAlloc((void**)&s->report_host, sizeof(int) * report_words(W), cudaHostAllocDefault));
   CKC(cudaStreamCreateWithFlags(&s->cap_stream, cudaStreamNonBlocking));
   CKC(cudaStreamCreateWithFlags(&s->body_stream, cudaStreamNonBlocking));
   CKC(cudaMalloc(&s->body_runs, 2 * sizeof(unsigned long long)));
@@ -1402,6 +1411,8 @@ void adf_destroy(adf_solver* s) {
                   (void*)s->pg_vel_d})
     if (p) cudaFree(p);
   if (s->pinned) cudaFreeHost(s->pinned);
+  if (s->report_dev) cudaFree(s->report_dev);
+  if (s->report_host) cudaFreeHost(s->report_host);
   if (s->list_entries) cudaFree(s->list_entries);
   if (s->body_runs) cudaFree(s->body_runs);
   if (s->perr) cudaFree(s->perr);
@@ -1566,14 +1577,7 @@ int adf_density_ratio(adf_solver* s, const float* q, const float* qd, float* rat
   P.qd = const_cast<float*>(qd);
   int rc = prepare(s, P, st);
   if (rc) return rc;
-  if (ratio_out) {
-    CK(cudaMemsetAsync(ratio_out, 0, sizeof(float) * s->n, st));
-    LAUNCH(s, k_unsort_n, blocks(s->n), BLOCK, st, s->n, P.nfw, P.id_of, P.ratio, 1, 0, ratio_out, 1);
-  }
-  if (active_out) {
-    CK(cudaMemsetAsync(active_out, 0, sizeof(float) * s->n, st));
-    LAUNCH(s, k_fill_ones, blocks(s->n), BLOCK, st, s->n, P.nfw, P.id_of, active_out);
-  }
+  if (ratio_out || active_out) LAUNCH(s, k_ratio_out, blocks(s->n), BLOCK, st, P, ratio_out, active_out);
   return check_launch();
 }
 
@@ -1583,42 +1587,57 @@ int adf_get_report(adf_solver* s, adf_report* r, void* stream) {
   const cudaStream_t st = (cudaStream_t)stream;
   const int W = s->W;
   if (W == 0) return cudaStreamSynchronize(st) == cudaSuccess ? ADF_OK : fail(ADF_ERR_CUDA, "adf_get_report: sync");
-  // every copy is ordered on the caller's stream (never the legacy default stream, which would wait for the work of
-  // other streams too); one synchronisation at the end
-  auto cp = [&](void* dst, const void* src, size_t bytes) -> int {
-    if (!dst) return ADF_OK;
-    CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
-    return ADF_OK;
+  // The asked-for arrays and the status words, packed on the device and read back in one copy ordered on the caller's
+  // stream (never the legacy default stream, which would wait for the work of other streams too): a copy an array, from
+  // pageable memory, cost a report of one world 200 us.
+  struct Field {
+    void* dst;
+    const void* src;
+    size_t bytes;
   };
-  int rc = 0;
-  rc |= cp(r->density_err, s->den_err, 4 * W);
-  rc |= cp(r->divergence_err, s->div_err, 4 * W);
-  rc |= cp(r->iters_density, s->iters_den, 4 * W);
-  rc |= cp(r->iters_divergence, s->iters_div, 4 * W);
-  rc |= cp(r->mass_in, s->mass_in, 8 * W);
-  rc |= cp(r->mass_out, s->d.mass_out, 8 * W);
-  rc |= cp(r->mass_initial, s->mass0, 8 * W);
-  rc |= cp(r->escaped, s->d.escaped, 4 * W);
-  rc |= cp(r->neighbor_overflow, s->d.overflow, 4 * W);
-  rc |= cp(r->max_speed, s->d.max_speed_bits, 4 * W);
-  rc |= cp(r->density_err_max, s->den_err_max, 4 * W);
-  rc |= cp(r->projected, s->d.projected, 4 * W);
-  rc |= cp(r->nonfinite, s->d.nonfinite, 4 * W);
-  rc |= cp(r->emitter_overflow, s->emit_overflow, 4 * W);
-  rc |= cp(r->density_tol, s->den_tol, 4 * W);
-  rc |= cp(r->swept, s->d.swept, 4 * W);
-  if (s->warm_alloc) {
-    rc |= cp(r->learned_divergence, s->d.learned, 4 * W);
-    rc |= cp(r->learned_density, s->d.learned + W, 4 * W);
-  } else {
-    if (r->learned_divergence) std::memset(r->learned_divergence, 0, 4 * (size_t)W);
-    if (r->learned_density) std::memset(r->learned_density, 0, 4 * (size_t)W);
-  }
-  if (rc) return ADF_ERR_CUDA;
   int merr = 0, perr = 0;
-  if (s->merr) CK(cudaMemcpyAsync(&merr, s->merr, sizeof(int), cudaMemcpyDeviceToHost, st));
-  if (s->perr) CK(cudaMemcpyAsync(&perr, s->perr, sizeof(int), cudaMemcpyDeviceToHost, st));
+  const size_t w4 = 4 * (size_t)W, w8 = 8 * (size_t)W;
+  const Field all[] = {{r->mass_in, s->mass_in, w8},
+                       {r->mass_out, s->d.mass_out, w8},
+                       {r->mass_initial, s->mass0, w8},
+                       {r->density_err, s->den_err, w4},
+                       {r->divergence_err, s->div_err, w4},
+                       {r->iters_density, s->iters_den, w4},
+                       {r->iters_divergence, s->iters_div, w4},
+                       {r->escaped, s->d.escaped, w4},
+                       {r->neighbor_overflow, s->d.overflow, w4},
+                       {r->max_speed, s->d.max_speed_bits, w4},
+                       {r->density_err_max, s->den_err_max, w4},
+                       {r->projected, s->d.projected, w4},
+                       {r->nonfinite, s->d.nonfinite, w4},
+                       {r->emitter_overflow, s->emit_overflow, w4},
+                       {r->density_tol, s->den_tol, w4},
+                       {r->swept, s->d.swept, w4},
+                       {r->learned_divergence, s->warm_alloc ? s->d.learned : nullptr, w4},
+                       {r->learned_density, s->warm_alloc ? s->d.learned + W : nullptr, w4},
+                       {&merr, s->merr, sizeof(int)},
+                       {&perr, s->perr, sizeof(int)}};
+  static_assert(sizeof(all) / sizeof(all[0]) <= ReportSrc::MAX, "report fields");
+  ReportSrc R{};
+  int fields = 0, words = 0;
+  for (const Field& f : all) {
+    if (!f.dst) continue;
+    if (!f.src) {
+      std::memset(f.dst, 0, f.bytes);
+      continue;
+    }
+    R.src[fields] = (const int*)f.src;
+    R.words[fields] = (int)(f.bytes / 4);
+    R.offset[fields++] = words;
+    words += (int)(f.bytes / 4);
+  }
+  std::lock_guard<std::mutex> lock(s->report_mutex);  // the staging buffers serve one reader at a time
+  LAUNCH(s, k_report_pack, dim3(std::min(blocks(2 * (long long)W), 64), fields), BLOCK, st, R, s->report_dev);
+  CK(cudaMemcpyAsync(s->report_host, s->report_dev, sizeof(int) * (size_t)words, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
+  fields = 0;
+  for (const Field& f : all)
+    if (f.dst && f.src) std::memcpy(f.dst, s->report_host + R.offset[fields++], f.bytes);
   if (merr) return fail(ADF_ERR_STATE, "warm-start network: a tensor-core wait expired; the learned starts are invalid");
   if (perr)
     return fail(ADF_ERR_STATE, "pressure solve: a grid-barrier wait of the persistent CG solve expired; the step's "
@@ -1904,8 +1923,10 @@ int adf_active_mass(adf_solver* s, int64_t* out_host, void* stream) {
   const int W = std::max(s->W, 1);
   CK(cudaMemsetAsync(s->tmp_mass, 0, 8 * W, st));
   if (s->n > 0) LAUNCH(s, k_active_mass, blocks(s->n), BLOCK, st, s->d, s->tmp_mass);
-  if (s->W) CK(cudaMemcpyAsync(out_host, s->tmp_mass, 8 * s->W, cudaMemcpyDeviceToHost, st));
+  std::lock_guard<std::mutex> lock(s->report_mutex);
+  if (s->W) CK(cudaMemcpyAsync(s->report_host, s->tmp_mass, 8 * s->W, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
+  if (s->W) std::memcpy(out_host, s->report_host, 8 * (size_t)s->W);
   return check_launch();
 }
 

@@ -3675,18 +3675,37 @@ __global__ void k_active_mass(DevP P, long long* out) {
   }
 }
 
+// density_ratio's outputs in the caller's order, every particle written once: the ratio and 1 of a liquid particle (its key
+// of the last sort is in the liquid's cells), 0 and 0 of any other; either may be null.
+__global__ void k_ratio_out(DevP P, float* ratio, float* active) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= P.n) return;
+  const int key = P.key_of[i];
+  const bool liquid = key >= 0 && key < P.total_cells;
+  if (ratio) ratio[i] = liquid ? P.ratio[P.pos_of[i]] : 0.0f;
+  if (active) active[i] = liquid ? 1.0f : 0.0f;
+}
+
+// The per-world arrays of a report side by side, in 4-byte words (block row: one array).
+struct ReportSrc {
+  static constexpr int MAX = 20;
+  const int* src[MAX];
+  int words[MAX];   // per array
+  int offset[MAX];  // in the packed words
+};
+
+__global__ void k_report_pack(const __grid_constant__ ReportSrc R, int* out) {
+  const int f = blockIdx.y;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < R.words[f]; k += gridDim.x * blockDim.x)
+    out[R.offset[f] + k] = R.src[f][k];
+}
+
 __global__ void k_unsort_n(int n, const int* nfw, const int* id_of, const float* f, int stride, int comp, float* out,
                            int ncomp) {
   int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n || p >= nfw[0]) return;
   int i = id_of[p];
   for (int c = 0; c < ncomp; ++c) out[ncomp * i + c] = f[(size_t)stride * p + comp + c];
-}
-
-__global__ void k_fill_ones(int n, const int* nfw, const int* id_of, float* out) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n || p >= nfw[0]) return;
-  out[id_of[p]] = 1.0f;
 }
 
 __global__ void k_count_entries(int n, const int* nfw, const int* cnt, long long* out) {

@@ -396,11 +396,16 @@ class SolverDFSPH:
         """Density ratio rho/rho0 of every particle of ``state`` and the active-liquid mask (solver.py:386-393)."""
         if self.n == 0:
             return np.zeros(0), np.zeros(0, dtype=bool)
-        ratio = torch.zeros(self.n, dtype=torch.float32, device=self.device)
-        active = torch.zeros(self.n, dtype=torch.float32, device=self.device)
+        n = self.n
+        # one buffer and one copy to the host: the ratios, then the mask as bytes (converted on the device)
+        buf = torch.empty(5 * n, dtype=torch.uint8, device=self.device)
+        ratio, mask = buf[:4 * n].view(torch.float32), buf[4 * n:].view(torch.bool)
+        active = torch.empty(n, dtype=torch.float32, device=self.device)
         _lib.check(self._lib.adf_density_ratio(self._h, _ptr(state.particle_q), _ptr(state.particle_qd),
                                                ratio.data_ptr(), active.data_ptr(), self._stream()), "density_ratio")
-        return ratio.cpu().numpy(), active.cpu().numpy() > 0.0
+        torch.gt(active, 0.0, out=mask)
+        host = buf.cpu().numpy()
+        return host[:4 * n].view(np.float32), host[4 * n:].view(np.bool_)
 
     def neighbor_rows(self) -> tuple[np.ndarray, np.ndarray]:
         """The last lists as global particle ids [n, capacity] (-1 past count) and counts (neighbors.py:285-295)."""
