@@ -203,6 +203,7 @@ struct adf_solver {
   bool cg_team = false;  // CG products by teams of TL lanes per particle (models of at most CG_TEAM_MAX particles)
   // whole solves as one cooperative launch (dfsph_group.cuh)
   int persist = -1;          // adf_set_persistent: 1, 0, or -1 (never called): grid_solves
+  int sms = 148;             // the device's multiprocessors
   int grid_blocks = 0;       // blocks of the launch (0: none)
   int grid_threads = 0;      // threads of each
   int least_priority = 0;
@@ -495,7 +496,9 @@ int prepare(adf_solver* s, DevP& P, cudaStream_t st) {
   }
   prof_end(s, st);
   prof_begin(s, 2, st);
-  LAUNCH(s, k_wall_slots, blocks(n), BLOCK, st, P);
+  // small blocks while BLOCK particles each would be fewer blocks than two per SM
+  if (blocks(n) < 2 * s->sms) LAUNCH(s, k_wall_slots<BLOCK / WT>, blocks(n, BLOCK / WT), BLOCK, st, P);
+  else LAUNCH(s, k_wall_slots<BLOCK>, blocks(n), BLOCK, st, P);
   if (P.slot_cap > 1) LAUNCH(s, k_shape_slots, blocks(n), BLOCK, st, P);
   prof_end(s, st);
   prof_begin(s, 3, st);
@@ -661,11 +664,11 @@ int grid_solve(adf_solver* s, const DevP& P, int mode, int init, cudaStream_t st
 // per SM their rows fit the SMs' shared memory (dfsph_small.cuh). Above, a thread each while the device holds that many:
 // every SM gets an even share. Above that, the form that takes fewer rounds (dfsph_group.cuh).
 int setup_grid_solve(adf_solver* s, int sph) {
+  CK(cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, s->device));
+  const int sms = s->sms;
   const long long runs = (long long)s->n / RUN + s->W;
   if (s->W == 0 || s->n == 0 || s->W > LIST_MAX_WORLDS || runs > LIST_MAX_ITEMS || s->d.n_chunks > LIST_MAX_ITEMS)
     return ADF_OK;
-  int sms = 0;
-  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
   int greatest = 0;
   CK(cudaDeviceGetStreamPriorityRange(&s->least_priority, &greatest));
   const long long deep = (long long)sms * GRID_BLOCK, wide = 2ll * sms * WIDE_BLOCK, n = std::max(sph, 1);

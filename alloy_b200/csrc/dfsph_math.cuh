@@ -106,6 +106,20 @@ __device__ __forceinline__ void wf(const KC& k, float r2, float& W, float& F) {
   if (r <= k.r_min) F = 0.0f;
 }
 
+// wf's W alone, without the divisions of F.
+__device__ __forceinline__ float kernel_w(const KC& k, float r2) {
+  const float q = __fmul_rn(__fsqrt_rn(r2), k.inv_h);
+  if (q >= 1.0f) return 0.0f;
+  if (k.kind == 0) {
+    if (q <= 0.5f) return __fmul_rn(k.sigma, ADF_FMA(__fmul_rn(6.0f, __fmul_rn(q, q)), __fsub_rn(q, 1.0f), 1.0f));
+    const float s = __fsub_rn(1.0f, q);
+    return __fmul_rn(k.sigma, __fmul_rn(2.0f, __fmul_rn(__fmul_rn(s, s), s)));
+  }
+  const float s = __fsub_rn(1.0f, q);
+  const float s2 = __fmul_rn(s, s);
+  return __fmul_rn(k.sigma, __fmul_rn(__fmul_rn(s2, s2), ADF_FMA(4.0f, q, 1.0f)));
+}
+
 // Psi(d) and dPsi/dd of a flat solid half-space at signed distance d (kernels.py:80-138, curvature 0).
 __device__ __forceinline__ void halfspace(const KC& k, float d, float& psi, float& dpsi) {
   if (d >= k.h) { psi = 0.0f; dpsi = 0.0f; return; }
