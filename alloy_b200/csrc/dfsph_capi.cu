@@ -209,7 +209,7 @@ struct adf_solver {
   int least_priority = 0;
   int grid_form = 0;         // 0 rows in shared memory (dfsph_small.cuh), 1 deep blocks, 2 wide (dfsph_group.cuh)
   int solve_runs = 0;                     // capacity of a list of runs
-  int* solve_ctr = nullptr;  // [2][CT_SIZE], one set per solve of a step (zeroed with the sort)
+  int* solve_ctr = nullptr;  // [3][CT_SIZE]: one set per solve of a step, one for the barriers between them
   int2* solve_items = nullptr;                          // [2][solve_runs]
   int *solve_chunks = nullptr, *solve_worlds = nullptr;  // [2][n_chunks], [2][W]
   // item halos of the pressure iterations (adf_set_halo): -1 the tuner times both forms, 0 off (the default), 1 always
@@ -464,7 +464,7 @@ void set_solve_params(adf_solver* s, DevP& P, int mode, double dt) {
   P.relief = (mode == 1 && p.relief_speed > 0.0) ? (float)(p.relief_speed * dt * p.lattice_grad) : (float)(1.0e30);
 }
 
-int prepare(adf_solver* s, DevP& P, cudaStream_t st) {
+int prepare(adf_solver* s, DevP& P, cudaStream_t st, bool density = true) {
   const int n = s->n;
   prof_begin(s, 0, st);
   if (P.skin_on) {  // which worlds rebuild their superset rows (dfsph_skin.cuh)
@@ -501,6 +501,10 @@ int prepare(adf_solver* s, DevP& P, cudaStream_t st) {
   else LAUNCH(s, k_wall_slots<BLOCK>, blocks(n), BLOCK, st, P);
   if (P.slot_cap > 1) LAUNCH(s, k_shape_slots, blocks(n), BLOCK, st, P);
   prof_end(s, st);
+  if (!density) {
+    s->built = true;
+    return check_launch();
+  }
   prof_begin(s, 3, st);
   run_tk(s, TK_DENSITY, st, P);
   prof_end(s, st);
@@ -623,14 +627,22 @@ const void* grid_kernel(const adf_solver* s) {
   return table[s->grid_form * 8 + (s->d.slot_cap > 1 ? 4 : 0) + (s->cg ? 2 : 0) + (s->W == 1 ? 1 : 0)];
 }
 
-// One solve (or, with init 0, its iterations and apply) in one launch.
-int grid_solve(adf_solver* s, const DevP& P, int mode, int init, cudaStream_t st) {
+const void* small_step_kernel(const adf_solver* s) {
+  static const void* const table[] = {
+      (const void*)k_small_step<false, false, false>, (const void*)k_small_step<false, false, true>,
+      (const void*)k_small_step<false, true, false>,  (const void*)k_small_step<false, true, true>,
+      (const void*)k_small_step<true, false, false>,  (const void*)k_small_step<true, false, true>,
+      (const void*)k_small_step<true, true, false>,   (const void*)k_small_step<true, true, true>};
+  return table[(s->d.slot_cap > 1 ? 4 : 0) + (s->cg ? 2 : 0) + (s->W == 1 ? 1 : 0)];
+}
+
+SolveArgs solve_args(const adf_solver* s, int mode, int init) {
   SolveArgs A{};
   A.init = init;
   A.ctr = s->solve_ctr + mode * CT_SIZE;
   for (int k = 0; k < 2; ++k) {
     A.items[k] = s->solve_items + (size_t)k * s->solve_runs;
-    A.chunks[k] = s->solve_chunks + (size_t)k * P.n_chunks;
+    A.chunks[k] = s->solve_chunks + (size_t)k * s->d.n_chunks;
     A.worlds[k] = s->solve_worlds + (size_t)k * s->W;
   }
   A.extra = s->persist_extra;
@@ -639,7 +651,10 @@ int grid_solve(adf_solver* s, const DevP& P, int mode, int init, cudaStream_t st
   A.iters_out = mode == 0 ? s->iters_div : s->iters_den;
   A.mean_out = mode == 0 ? s->div_err : s->den_err;
   A.max_out = mode == 0 ? nullptr : s->den_err_max;
-  CK(cudaMemsetAsync(A.ctr, 0, sizeof(int) * CT_SIZE, st));
+  return A;
+}
+
+int launch_resident(adf_solver* s, const void* kernel, void** args, cudaStream_t st) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)s->grid_blocks);
   cfg.blockDim = dim3((unsigned)s->grid_threads);
@@ -654,10 +669,23 @@ int grid_solve(adf_solver* s, const DevP& P, int mode, int init, cudaStream_t st
   at[1].val.priority = s->least_priority;
   cfg.attrs = at;
   cfg.numAttrs = 2;
-  void* args[] = {const_cast<DevP*>(&P), &A};
-  CK(cudaLaunchKernelExC(&cfg, grid_kernel(s), args));
+  CK(cudaLaunchKernelExC(&cfg, kernel, args));
   ++s->launches;
   return ADF_OK;
+}
+
+// One solve (or, with init 0, its iterations and apply) in one launch.
+int grid_solve(adf_solver* s, const DevP& P, int mode, int init, cudaStream_t st) {
+  SolveArgs A = solve_args(s, mode, init);
+  CK(cudaMemsetAsync(A.ctr, 0, sizeof(int) * CT_SIZE, st));
+  void* args[] = {const_cast<DevP*>(&P), &A};
+  return launch_resident(s, grid_kernel(s), args, st);
+}
+
+// Whether everything after the rows and walls of this step is one launch (k_small_step): the small form, both solves
+// whole (no learned start, whose network runs between, and no feature record).
+bool step_in_one(const adf_solver* s, const DevP& P) {
+  return s->grid_form == 0 && grid_solves(s, P) && !s->tuning && s->prm.divergence_solve && !s->warm_on && !s->feat_rec;
 }
 
 // Shape of the cooperative launch, from the particles that are or can become liquid (`sph`). Up to SMALL_BLOCK of them
@@ -691,11 +719,18 @@ int setup_grid_solve(adf_solver* s, int sph) {
   if (smem) CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per_sm = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, s->grid_threads, smem));
+  if (s->grid_form == 0) {
+    const void* step = small_step_kernel(s);
+    int step_sm = 0;
+    CK(cudaFuncSetAttribute(step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&step_sm, step, s->grid_threads, smem));
+    per_sm = std::min(per_sm, step_sm);
+  }
   if ((long long)per_sm * sms < s->grid_blocks) {  // not all resident: one kernel per phase
     s->grid_blocks = 0;
     return ADF_OK;
   }
-  int rc = s->alloc(&s->solve_ctr, 2 * CT_SIZE) | s->alloc(&s->solve_items, 2 * (size_t)runs) |
+  int rc = s->alloc(&s->solve_ctr, 3 * CT_SIZE) | s->alloc(&s->solve_items, 2 * (size_t)runs) |
            s->alloc(&s->solve_chunks, 2 * (size_t)std::max(s->d.n_chunks, 1)) | s->alloc(&s->solve_worlds, 2 * (size_t)s->W);
   return rc ? ADF_ERR_CUDA : ADF_OK;
 }
@@ -812,12 +847,29 @@ mlp::Net solver_net(const adf_solver* s) {
   return mlp::Net{s->mw1, s->mw2, s->mparams, s->mnorm, s->merr, mlp::WAIT_LIMIT};
 }
 
+// This step's density tolerance per world (solve_driver.py:99-110), from the last step's density warm starts.
+int density_tolerance(adf_solver* s, DevP& P, double dt, cudaStream_t st) {
+  const int W = s->W;
+  if (P.n_chunks > 0) {
+    LAUNCH(s, k_jitter_chunks, (P.n_chunks + 7) / 8, 256, st, P, 1, s->jit_part);
+    LAUNCH(s, k_jitter_worlds, (W + 7) / 8, 256, st, P, 1, (const double*)s->jit_part, s->jit_head);
+  } else {
+    CK(cudaMemsetAsync(s->jit_head, 0, sizeof(double) * JIT_TERMS * W, st));
+  }
+  const adf_params& p = s->prm;
+  LAUNCH(s, k_tol_scale, blocks(W), BLOCK, st, P, (const double*)s->jit_head,
+         p.jitter_ratio > 0.0 ? (const double*)s->jit_flow : nullptr, (float)dt, (float)p.jitter_speed,
+         (float)p.jitter_ratio, (float)p.tol_den, (float)p.tol_den_min, s->jit_scale, s->den_tol);
+  return ADF_OK;
+}
+
 // pressure.py:355-390 + solve_driver.py:121-186 (Jacobi branch) + pressure.py:393-480
 int solve(adf_solver* s, DevP& P, int mode, double dt, cudaStream_t st, bool graph) {
   set_solve_params(s, P, mode, dt);
   const int n = s->n, W = s->W;
   const bool first = mode == 0 || !s->prm.divergence_solve;  // the step's first solve records the features
   const bool warm = s->warm_on && W > 0;
+  int rc = ADF_OK;
   const bool grid = grid_solves(s, P);
   const bool whole = grid && !warm && !(first && s->feat_rec);  // the start too is the group launch's
   if (!whole) {
@@ -830,17 +882,9 @@ int solve(adf_solver* s, DevP& P, int mode, double dt, cudaStream_t st, bool gra
   const bool subset = warm && first && s->judge && !s->cg && !s->feat_rec;
   P.warm_need = subset ? s->warm_need : nullptr;
   if (subset) LAUNCH(s, k_warm_need, blocks(W), BLOCK, st, P, s->warm_need);
-  if (mode == 1 && s->jit_scale && W > 0) {  // this step's density tolerance per world (solve_driver.py:99-110)
-    if (P.n_chunks > 0) {
-      LAUNCH(s, k_jitter_chunks, (P.n_chunks + 7) / 8, 256, st, P, 1, s->jit_part);
-      LAUNCH(s, k_jitter_worlds, (W + 7) / 8, 256, st, P, 1, (const double*)s->jit_part, s->jit_head);
-    } else {
-      CK(cudaMemsetAsync(s->jit_head, 0, sizeof(double) * JIT_TERMS * W, st));
-    }
-    const adf_params& p = s->prm;
-    LAUNCH(s, k_tol_scale, blocks(W), BLOCK, st, P, (const double*)s->jit_head,
-           p.jitter_ratio > 0.0 ? (const double*)s->jit_flow : nullptr, (float)dt, (float)p.jitter_speed,
-           (float)p.jitter_ratio, (float)p.tol_den, (float)p.tol_den_min, s->jit_scale, s->den_tol);
+  if (mode == 1 && s->jit_scale && W > 0) {
+    rc = density_tolerance(s, P, dt, st);
+    if (rc) return rc;
   }
   if (whole) return grid_solve(s, P, mode, 1, st);
   prof_begin(s, 4, st);
@@ -869,7 +913,7 @@ int solve(adf_solver* s, DevP& P, int mode, double dt, cudaStream_t st, bool gra
   } else {
     CK(cudaMemsetAsync(P.n_cw, 0, sizeof(int), st));
   }
-  int rc = check_launch();
+  rc = check_launch();
   if (rc) return rc;
   const bool dual = warm && s->judge && !s->cg;  // the first-sweep judge is a Jacobi sweep
   if (dual) dual_iteration(s, P, st);
@@ -1450,27 +1494,47 @@ int enqueue_step(adf_solver* s, const float* q_in, const float* qd_in, float* q_
   P.n_sinks = (int)s->sinks_h.size();
   P.sinks = s->sinks_d;
   CK(cudaMemsetAsync(P.max_speed_bits, 0, sizeof(int) * std::max(s->W, 1), st));
-  int rc = prepare(s, P, st);
+  const bool one = step_in_one(s, P);
+  int rc = prepare(s, P, st, !one);
   if (rc) return rc;
   if (s->jit_scale && s->prm.jitter_ratio > 0.0 && P.n_chunks > 0) {  // the liquid's mean start velocity per world
     LAUNCH(s, k_jitter_chunks, (P.n_chunks + 7) / 8, 256, st, P, 0, s->jit_part);
     LAUNCH(s, k_jitter_worlds, (s->W + 7) / 8, 256, st, P, 0, (const double*)s->jit_part, s->jit_flow);
   }
-  if (s->prm.divergence_solve) {
-    rc = solve(s, P, 0, dt, st, graph);
+  if (one) {
+    if (s->jit_scale) {
+      rc = density_tolerance(s, P, dt, st);
+      if (rc) return rc;
+    }
+    set_solve_params(s, P, 0, dt);
+    P.feat_on = 0;
+    DevP D = P;
+    std::swap(D.vel, D.vel2);
+    set_solve_params(s, D, 1, dt);
+    SolveArgs A = solve_args(s, 0, 1), B = solve_args(s, 1, 1);
+    int* between = s->solve_ctr + 2 * CT_SIZE;
+    CK(cudaMemsetAsync(s->solve_ctr, 0, sizeof(int) * 3 * CT_SIZE, st));
+    void* args[] = {&P, &D, &A, &B, &between};
+    rc = launch_resident(s, small_step_kernel(s), args, st);
     if (rc) return rc;
+    std::swap(P.vel, P.vel2);
+  } else {
+    if (s->prm.divergence_solve) {
+      rc = solve(s, P, 0, dt, st, graph);
+      if (rc) return rc;
+    }
+    P.dt = (float)dt;
+    prof_begin(s, 9, st);
+    run_tk(s, TK_XSPH, st, P);
+    prof_end(s, st);
+    std::swap(P.vel, P.vel2);
+    rc = solve(s, P, 1, dt, st, graph);
+    if (rc) return rc;
+    prof_begin(s, 10, st);
+    MS_DISPATCH(k_finish, blocks(s->n), BLOCK, st, P);
+    ++s->launches;
+    prof_end(s, st);
   }
-  P.dt = (float)dt;
-  prof_begin(s, 9, st);
-  run_tk(s, TK_XSPH, st, P);
-  prof_end(s, st);
-  std::swap(P.vel, P.vel2);
-  rc = solve(s, P, 1, dt, st, graph);
-  if (rc) return rc;
-  prof_begin(s, 10, st);
-  MS_DISPATCH(k_finish, blocks(s->n), BLOCK, st, P);
-  ++s->launches;
-  prof_end(s, st);
   const int ne = (int)s->em_h.size();
   if (ne > 0) {
     prof_begin(s, 11, st);

@@ -1671,12 +1671,38 @@ __device__ __forceinline__ void next_batch(int (&j)[NB], float (&f)[NB], const i
 
 // ------------------------------------------------------------------------------------------ density, factor
 // pressure.py:144-193
+// Particle p's density ratio, factor, neighbour count and compliance from its row's sums and its walls.
+template <bool MS>
+__device__ __forceinline__ void density_finish(const DevP& P, int p, int c, float inv_r0, float rho, float Gx, float Gy,
+                                               float Gz, float sq) {
+  float psi = 0.0f, lam = 0.0f;  // boundary slots, nearest first; lam: the opposing-wall compliance
+  for_slots<MS>(P, p, [&](int b, size_t o) {
+    const float4 sg = P.slot_g[o];
+    psi = psi + sg.w;
+    Gx = Gx + sg.x;
+    Gy = Gy + sg.y;
+    Gz = Gz + sg.z;
+    if constexpr (MS) {
+      const int ns = P.slot_cnt[p];
+      for (int c = b + 1; c < ns; ++c) {
+        const float4 gc = P.slot_g[slot_at(P, c, p)];
+        lam = lam + maxr(-2.0f * dot_plain(sg.x, sg.y, sg.z, gc.x, gc.y, gc.z), 0.0f);
+      }
+    }
+  });
+  float tot = (dotf(Gx, Gy, Gz, Gx, Gy, Gz) + sq) + lam;
+  lam = lam + maxr(P.tot_min - tot, 0.0f);
+  tot = maxr(tot, P.tot_min);
+  P.reg[p] = lam;
+  P.ratio[p] = ADF_FMA(rho, inv_r0, psi);
+  P.alpha[p] = (tot > (float)(1.0e-12)) ? 1.0f / tot : 0.0f;
+  P.neff[p] = ADF_FMA(psi, P.n_full, (float)c);
+}
+
 template <int NBX>
-__global__ void __launch_bounds__(BLOCK, 5) k_density_alpha(DevP P) {
+__device__ __forceinline__ void density_one(const DevP& P, int p) {
   constexpr int NB = NBX & NB_MASK;
   constexpr bool MS = (NBX & MS_FLAG) != 0;
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.nfw[0]) return;
   float4 xi = P.pos[p];
   float mi = xi.w;
   float inv_r0 = 1.0f / P.vel[p].w;
@@ -1710,28 +1736,13 @@ __global__ void __launch_bounds__(BLOCK, 5) k_density_alpha(DevP P) {
       sq = ADF_FMA(bi * a, (F * F) * r2, sq);
     }
   }
-  float psi = 0.0f, lam = 0.0f;  // boundary slots, nearest first; lam: the opposing-wall compliance
-  for_slots<MS>(P, p, [&](int b, size_t o) {
-    const float4 sg = P.slot_g[o];
-    psi = psi + sg.w;
-    Gx = Gx + sg.x;
-    Gy = Gy + sg.y;
-    Gz = Gz + sg.z;
-    if constexpr (MS) {
-      const int ns = P.slot_cnt[p];
-      for (int c = b + 1; c < ns; ++c) {
-        const float4 gc = P.slot_g[slot_at(P, c, p)];
-        lam = lam + maxr(-2.0f * dot_plain(sg.x, sg.y, sg.z, gc.x, gc.y, gc.z), 0.0f);
-      }
-    }
-  });
-  float tot = (dotf(Gx, Gy, Gz, Gx, Gy, Gz) + sq) + lam;
-  lam = lam + maxr(P.tot_min - tot, 0.0f);
-  tot = maxr(tot, P.tot_min);
-  P.reg[p] = lam;
-  P.ratio[p] = ADF_FMA(rho, inv_r0, psi);
-  P.alpha[p] = (tot > (float)(1.0e-12)) ? 1.0f / tot : 0.0f;
-  P.neff[p] = ADF_FMA(psi, P.n_full, (float)c);
+  density_finish<MS>(P, p, c, inv_r0, rho, Gx, Gy, Gz, sq);
+}
+
+template <int NBX>
+__global__ void __launch_bounds__(BLOCK, 5) k_density_alpha(DevP P) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < P.nfw[0]) density_one<NBX>(P, p);
 }
 
 // --------------------------------------------------------------------------------------------- solve start
@@ -3366,31 +3377,48 @@ __global__ void __launch_bounds__(BLOCK) k_apply(DevP P) {
 // integrate.py:150-178: gravity, external force, XSPH with Monaghan's symmetric weight m_j / rho_bar_ij.
 // The output array becomes the velocity array for the rest of the step (the host swaps them), so boundary
 // particles carry their own velocity across: the wall advance in k_finish reads it.
-template <int NBX>
-__global__ void __launch_bounds__(BLOCK, 3) k_xsph(DevP P) {
-  constexpr int NB = NBX & NB_MASK;
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  const int nf = P.nfw[0];
-  if (p >= nf) {
-    if (p < nf + P.nfw[1]) P.vel2[p] = P.vel[p];
-    return;
-  }
+// `sum(vi, rho_i, cx, cy, cz)`: the row's weighted velocity differences.
+template <class S>
+__device__ __forceinline__ void xsph_with(const DevP& P, int p, S sum) {
   const float dt = P.dt;
   float4 vi = P.vel[p];
   int w = P.world_s[p];
   float gx = P.gravity[3 * w], gy = P.gravity[3 * w + 1], gz = P.gravity[3 * w + 2];
-  float4 xi = P.pos[p];
   if (P.f_ext) {
     int i = P.id_of[p];
-    gx = gx + P.f_ext[3 * i] / xi.w;
-    gy = gy + P.f_ext[3 * i + 1] / xi.w;
-    gz = gz + P.f_ext[3 * i + 2] / xi.w;
+    const float m = P.pos[p].w;
+    gx = gx + P.f_ext[3 * i] / m;
+    gy = gy + P.f_ext[3 * i + 1] / m;
+    gz = gz + P.f_ext[3 * i + 2] / m;
   }
   float vx = ADF_FMA(dt, gx, vi.x), vy = ADF_FMA(dt, gy, vi.y), vz = ADF_FMA(dt, gz, vi.z);
   const float c = P.xsph_c;
   if (c > 0.0f) {
     float cx = 0.0f, cy = 0.0f, cz = 0.0f;
-    float rho_i = P.ratio[p] * vi.w;
+    sum(vi, P.ratio[p] * vi.w, cx, cy, cz);
+    vx = ADF_FMA(c, cx, vx);
+    vy = ADF_FMA(c, cy, vy);
+    vz = ADF_FMA(c, cz, vz);
+  }
+  P.vel2[p] = make_float4(vx, vy, vz, vi.w);
+}
+
+// One entry's term: Monaghan's symmetric weight m_j / rho_bar_ij of the velocity difference.
+__device__ __forceinline__ void xsph_term(const float4& vi, float rho_i, const float4& vj, float ratio_j, float mj, float W,
+                                          float& cx, float& cy, float& cz) {
+  float rho_bar = 0.5f * (rho_i + ratio_j * vj.w);
+  if (rho_bar > 0.0f) {
+    float cw = (mj / rho_bar) * W;  // W(r_ij) as the density pass evaluated it for this entry
+    cx = ADF_FMA(cw, vj.x - vi.x, cx);
+    cy = ADF_FMA(cw, vj.y - vi.y, cy);
+    cz = ADF_FMA(cw, vj.z - vi.z, cz);
+  }
+}
+
+template <int NBX>
+__device__ __forceinline__ void xsph_one(const DevP& P, int p) {
+  constexpr int NB = NBX & NB_MASK;
+  xsph_with(P, p, [&](const float4& vi, float rho_i, float& cx, float& cy, float& cz) {
     int cn = P.cnt[p];
     for (int k = 0; k < cn; k += NB) {
       int j[NB];
@@ -3409,21 +3437,18 @@ __global__ void __launch_bounds__(BLOCK, 3) k_xsph(DevP P) {
 #pragma unroll
       for (int u = 0; u < NB; ++u) {
         if (k + u >= cn) break;
-        float4 vj = vb[u];
-        float rho_bar = 0.5f * (rho_i + rb[u] * vj.w);
-        if (rho_bar > 0.0f) {
-          float cw = (mb[u] / rho_bar) * wb[u];  // W(r_ij) as k_density_alpha evaluated it for this entry
-          cx = ADF_FMA(cw, vj.x - vi.x, cx);
-          cy = ADF_FMA(cw, vj.y - vi.y, cy);
-          cz = ADF_FMA(cw, vj.z - vi.z, cz);
-        }
+        xsph_term(vi, rho_i, vb[u], rb[u], mb[u], wb[u], cx, cy, cz);
       }
     }
-    vx = ADF_FMA(c, cx, vx);
-    vy = ADF_FMA(c, cy, vy);
-    vz = ADF_FMA(c, cz, vz);
-  }
-  P.vel2[p] = make_float4(vx, vy, vz, vi.w);
+  });
+}
+
+template <int NBX>
+__global__ void __launch_bounds__(BLOCK, 3) k_xsph(DevP P) {
+  int p = blockIdx.x * blockDim.x + threadIdx.x;
+  const int nf = P.nfw[0];
+  if (p < nf) xsph_one<NBX>(P, p);
+  else if (p < nf + P.nfw[1]) P.vel2[p] = P.vel[p];
 }
 
 // ------------------------------------------------------------------------------------------------ finish
@@ -3564,11 +3589,9 @@ __device__ __forceinline__ void finish_walls(const DevP& P, int p, int w, float 
   if (moved) atomicAdd(&P.projected[w], 1);
 }
 
+// Sorted particle p, liquid or wall (nf: the liquid's count).
 template <bool MS>
-__global__ void __launch_bounds__(BLOCK) k_finish(DevP P) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  int nf = P.nfw[0];
-  if (p >= nf + P.nfw[1]) return;
+__device__ __forceinline__ void finish_one(const DevP& P, int p, int nf) {
   const float dt = P.dt;
   int i = P.id_of[p];
   float4 xi = P.pos[p];
@@ -3646,6 +3669,13 @@ __global__ void __launch_bounds__(BLOCK) k_finish(DevP P) {
   P.qd[3 * i + 2] = vz;
   P.kv[i] = P.kv_s[p];
   P.kd[i] = P.kd_s[p];
+}
+
+template <bool MS>
+__global__ void __launch_bounds__(BLOCK) k_finish(DevP P) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  const int nf = P.nfw[0];
+  if (p < nf + P.nfw[1]) finish_one<MS>(P, p, nf);
 }
 
 // ---------------------------------------------------------------------------------------------- emitters

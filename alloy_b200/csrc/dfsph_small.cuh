@@ -7,6 +7,10 @@
 // changes (kappa / rho0 or the direction, 4 bytes, for the acceleration; the acceleration, 16 bytes, for its
 // divergence), all gathers of a row in flight at once, instead of rows, positions and that value.
 //
+// A step of such a model is one launch after its rows and walls (k_small_step): density, both solves, XSPH and the finish
+// read the rows once. Against a launch for each: four steps of 2,016 particles 685 -> 624 us, of 8,000 with reports 1085
+// -> 1020, of the 30k column 2551 -> 2495, of the 30k tank 1964 -> 1910.
+//
 // What bounded these phases before: on 30,720 particles an acceleration or divergence phase took 7 to 9 us, 21 MB
 // through the L2 after every barrier's L1 invalidation, in eight dependent trips a thread.
 //
@@ -49,7 +53,7 @@ struct SmallSolve {
   __device__ __forceinline__ int warps() const { return threads() >> 5; }
   __device__ __forceinline__ int at(int k) const { return k * SMALL_BLOCK + threadIdx.x; }
 
-  // The row into shared memory, the walls' gradients into registers.
+  // The row into shared memory, as the density pass left it.
   __device__ __forceinline__ void load(const float4& xi) {
     const int m = min(c, ROW_RES);
     for (int k = 0; k < m; k += NB) {
@@ -66,6 +70,48 @@ struct SmallSolve {
           jm[at(k + u)] = make_int2(j[u], __float_as_int(x[u].w));
         }
     }
+    walls();
+  }
+
+  // The density pass (density_one) with the row kept; only entries past the resident ones are written out.
+  __device__ __forceinline__ void load_density(const float4& xi) {
+    const float inv_r0 = 1.0f / r0;
+    const float bi = xi.w * inv_r0;
+    float rho = xi.w * P.kc.sigma, Gx = 0.0f, Gy = 0.0f, Gz = 0.0f, sq = 0.0f;
+    for (int k = 0; k < c; k += NB) {
+      int j[NB];
+      load_row_batch(P, p, c, k, j);
+      float4 x[NB];
+#pragma unroll
+      for (int u = 0; u < NB; ++u) x[u] = P.pos[j[u]];
+#pragma unroll
+      for (int u = 0; u < NB; ++u)
+        if (k + u < c) {
+          const float rx = xi.x - x[u].x, ry = xi.y - x[u].y, rz = xi.z - x[u].z;
+          const float r2 = dot_plain(rx, ry, rz, rx, ry, rz);
+          float W, F;
+          wf(P.kc, r2, W, F);
+          if (k + u < ROW_RES) {
+            geo[at(k + u)] = make_float4(rx, ry, rz, F);
+            jm[at(k + u)] = make_int2(j[u], __float_as_int(x[u].w));
+          } else {
+            P.nbrjf[(size_t)(k + u) * P.n + p] = make_int2(j[u], __float_as_int(F));
+          }
+          rho = ADF_FMA(x[u].w, W, rho);
+          const float a = x[u].w * inv_r0;
+          const float aF = a * F;
+          Gx = ADF_FMA(aF, rx, Gx);
+          Gy = ADF_FMA(aF, ry, Gy);
+          Gz = ADF_FMA(aF, rz, Gz);
+          sq = ADF_FMA(bi * a, (F * F) * r2, sq);
+        }
+    }
+    density_finish<MS>(P, p, c, inv_r0, rho, Gx, Gy, Gz, sq);
+    walls();
+  }
+
+  // The walls' gradients into registers.
+  __device__ __forceinline__ void walls() {
     if constexpr (MS) {
       ns = P.slot_cnt[p];
 #pragma unroll
@@ -88,6 +134,7 @@ struct SmallSolve {
   template <class V, class G, class F>
   __device__ __forceinline__ void for_row(G gather, F f) {
     const int m = min(c, ROW_RES);
+#pragma unroll 1
     for (int k = 0; k < m; k += NB) {
       V v[NB];
       float mj[NB];
@@ -374,13 +421,12 @@ struct SmallSolve {
     return true;
   }
 
-  __device__ __forceinline__ void run() {
+  // This thread's particle: blocks take even shares of the liquid in whole warps.
+  __device__ __forceinline__ void place() {
     const int nf = P.nfw[0];
-    div = P.mode == 0;
-    dt = P.dt;
-    scale = div ? dt : dt * dt;
-    int it = 0;
-    bool open;
+    const int share = ((nf + (int)gridDim.x - 1) / (int)gridDim.x + 31) & ~31;
+    p = blockIdx.x * share + threadIdx.x;
+    mine = (int)threadIdx.x < share && p < nf;
     if constexpr (ONE) {
       const int2 r = P.wrange[0];
       n_one = r.y - r.x;
@@ -388,6 +434,22 @@ struct SmallSolve {
       ie = P.skin_ws[1];
       c0 = P.world_chunk_start[0];
       c1 = P.world_chunk_start[1];
+    }
+    if (mine) {
+      w = ONE ? 0 : P.world_s[p];
+      c = P.cnt[p];
+      id = P.id_of[p];
+      r0 = P.vel[p].w;
+    }
+  }
+
+  // The world's part of a solve's start (k_begin_solve) and the cleared residuals; `it` the iterations done before.
+  __device__ __forceinline__ void begin(int& it, bool& open) {
+    div = P.mode == 0;
+    dt = P.dt;
+    scale = div ? dt : dt * dt;
+    it = 0;
+    if constexpr (ONE) {
       open = n_one > 0 && (A.init || P.converged[0] == 0);
       if (!A.init) it = P.iters[0];
       else if (tid() == 0) {
@@ -397,7 +459,7 @@ struct SmallSolve {
       }
       if (P.iter_work && CG && open && tid() == 0) atomicAdd(P.iter_work, (unsigned long long)n_one);
     } else {
-      for (int v = tid(); v < P.W; v += threads()) {  // k_begin_solve
+      for (int v = tid(); v < P.W; v += threads()) {
         const int2 r = P.wrange[v];
         bool go = r.y > r.x;
         if (A.init) {
@@ -412,46 +474,43 @@ struct SmallSolve {
         if (CG && go && P.iter_work) atomicAdd(P.iter_work, (unsigned long long)(r.y - r.x));
       }
     }
-    // particles per block: an even share of the liquid in whole warps
-    const int share = ((nf + (int)gridDim.x - 1) / (int)gridDim.x + 31) & ~31;
-    p = blockIdx.x * share + threadIdx.x;
-    mine = (int)threadIdx.x < share && p < nf;
-    if (mine) {
-      const float4 xi = P.pos[p], vi = P.vel[p];
-      w = ONE ? 0 : P.world_s[p];
-      c = P.cnt[p];
-      id = P.id_of[p];
-      reg = P.reg[p];
-      alpha = P.alpha[p];
-      few = P.neff[p] < P.min_nb;
-      r0 = vi.w;
-      load(xi);
-      if (A.init) {
-        const float inv_r0 = 1.0f / r0;
-        float rate = 0.0f;
-        for_row<float4>([&](int j) { return P.vel[j]; },
-                        [&](const float4& vj, const float4& g, float mj) {
-                          const float aF = (mj * inv_r0) * g.w;
-                          rate = ADF_FMA(aF, dotf(vi.x - vj.x, vi.y - vj.y, vi.z - vj.z, g.x, g.y, g.z), rate);
-                        });
-#pragma unroll
-        for (int b = 0; b < NS; ++b)
-          if (b < ns) {
-            const float4 vb = P.slot_vb[slot_at(P, b, p)];
-            rate = rate + dotf(vi.x - vb.x, vi.y - vb.y, vi.z - vb.z, gx[b], gy[b], gz[b]);
-          }
-        solve_start(P, p, vi, rate, kap, lower, src);
-      } else {
-        kap = P.kappa[p];
-        lower = P.lower[p];
-        src = P.src[p];
-      }
-    }
     if (CG)
       for (int i = tid(); i < P.n; i += threads()) P.cg_pair[i] = make_float2(0.0f, 0.0f);
     if (A.init)
       for (int i = tid(); i < P.n; i += threads()) P.err_orig[i] = 0.0f;
-    if (!sync()) return;
+  }
+
+  // The particle's part (solve_init_one), its row resident.
+  __device__ __forceinline__ void start() {
+    reg = P.reg[p];
+    alpha = P.alpha[p];
+    few = P.neff[p] < P.min_nb;
+    if (A.init) {
+      const float4 vi = P.vel[p];
+      const float inv_r0 = 1.0f / r0;
+      float rate = 0.0f;
+      for_row<float4>([&](int j) { return P.vel[j]; },
+                      [&](const float4& vj, const float4& g, float mj) {
+                        const float aF = (mj * inv_r0) * g.w;
+                        rate = ADF_FMA(aF, dotf(vi.x - vj.x, vi.y - vj.y, vi.z - vj.z, g.x, g.y, g.z), rate);
+                      });
+#pragma unroll
+      for (int b = 0; b < NS; ++b)
+        if (b < ns) {
+          const float4 vb = P.slot_vb[slot_at(P, b, p)];
+          rate = rate + dotf(vi.x - vb.x, vi.y - vb.y, vi.z - vb.z, gx[b], gy[b], gz[b]);
+        }
+      solve_start(P, p, vi, rate, kap, lower, src);
+    } else {
+      kap = P.kappa[p];
+      lower = P.lower[p];
+      src = P.src[p];
+    }
+  }
+
+  // From the start on: the iterations, the velocity update and the statistics. False when a wait gave up.
+  __device__ __forceinline__ bool solve(int it, bool open) {
+    if (!sync()) return false;
     if constexpr (ONE) {
       on = mine && open;
     } else {
@@ -460,14 +519,14 @@ struct SmallSolve {
     }
     if (open) {
       if constexpr (CG) {
-        if (!cg(it)) return;
+        if (!cg(it)) return false;
       } else {
-        if (!jacobi(it)) return;
+        if (!jacobi(it)) return false;
       }
     }
     if (CG && open) {  // the solved kappa / rho0 for the neighbours' acceleration
       if (mine) P.kr[p] = kap / r0;
-      if (!sync()) return;
+      if (!sync()) return false;
     }
     if (mine) {
       P.kappa[p] = kap;
@@ -478,21 +537,127 @@ struct SmallSolve {
       A.mean_out[v] = P.err_mean[v];
       if (A.max_out) A.max_out[v] = P.emax[v];
     }
+    return true;
+  }
+
+  __device__ __forceinline__ void run() {
+    int it;
+    bool open;
+    place();
+    begin(it, open);
+    if (mine) {
+      load(P.pos[p]);
+      start();
+    }
+    solve(it, open);
+  }
+
+  // The step from its rows and walls on: density, divergence solve, XSPH (velocities into D.vel, the density solve's),
+  // density solve (parameters D and B), finish.
+  __device__ __forceinline__ void run_step(const DevP& D, const SolveArgs& B) {
+    int it;
+    bool open;
+    place();
+    begin(it, open);
+    if (mine) {
+      load_density(P.pos[p]);
+      start();
+    }
+    if (!solve(it, open)) return;
+    if (!sync()) return;
+    struct Other {
+      float4 v;
+      float ratio;
+    };
+    if (mine)
+      xsph_with(P, p, [&](const float4& vi, float rho_i, float& cx, float& cy, float& cz) {
+        for_row<Other>([&](int j) { return Other{P.vel[j], P.ratio[j]}; },
+                       [&](const Other& o, const float4& g, float mj) {
+                         xsph_term(vi, rho_i, o.v, o.ratio, mj, kernel_w(P.kc, dot_plain(g.x, g.y, g.z, g.x, g.y, g.z)), cx,
+                                   cy, cz);
+                       });
+      });
+    const int nf = P.nfw[0], all = nf + P.nfw[1];
+    for (int q = nf + tid(); q < all; q += threads()) P.vel2[q] = P.vel[q];
+    if (!sync()) return;
+    SmallSolve d{D, B, sync, geo, jm};
+    d.p = p;
+    d.w = w;
+    d.c = c;
+    d.id = id;
+    d.mine = mine;
+    d.r0 = r0;
+    d.ns = ns;
+#pragma unroll
+    for (int b = 0; b < NS; ++b) {
+      d.gx[b] = gx[b];
+      d.gy[b] = gy[b];
+      d.gz[b] = gz[b];
+    }
+    d.c0 = c0;
+    d.c1 = c1;
+    d.ib = ib;
+    d.ie = ie;
+    d.n_one = n_one;
+    d.begin(it, open);
+    if (mine) d.start();
+    if (!d.solve(it, open)) return;
+    if (mine) finish_one<MS>(D, p, nf);
+    for (int q = nf + tid(); q < all; q += threads()) finish_one<MS>(D, q, nf);
   }
 };
+
+// The solve when the liquid outgrew the blocks: particles that were no liquid at creation became liquid since. Out of
+// line, so that the kernels below carry neither its code nor its registers.
+template <bool MS, bool CG, bool ONE>
+__device__ __noinline__ void outgrown_solve(const DevP& P, const SolveArgs& A) {
+  GridSolve<MS, CG, ONE> g{P, A, GridSync{0u, gridDim.x + A.extra, A.ctr + CT_ARRIVE, A.status, A.wait_limit}};
+  g.run();
+}
 
 template <bool MS, bool CG, bool ONE>
 __global__ void __launch_bounds__(SMALL_BLOCK, 1)
 k_small_solve(const __grid_constant__ DevP P, const __grid_constant__ SolveArgs A) {
   extern __shared__ float4 small_rows[];
-  if (P.nfw[0] > (int)gridDim.x * SMALL_BLOCK) {  // particles that were no liquid at creation became liquid since
-    GridSolve<MS, CG, ONE> g{P, A, GridSync{0u, gridDim.x + A.extra, A.ctr + CT_ARRIVE, A.status, A.wait_limit}};
-    g.run();
+  if (P.nfw[0] > (int)gridDim.x * SMALL_BLOCK) {
+    outgrown_solve<MS, CG, ONE>(P, A);
     return;
   }
   SmallSolve<MS, CG, ONE> g{P, A, GridSync{0u, gridDim.x + A.extra, A.ctr + CT_ARRIVE, A.status, A.wait_limit}, small_rows,
                             reinterpret_cast<int2*>(small_rows + ROW_RES * SMALL_BLOCK)};
   g.run();
+}
+
+// Everything of a step after its neighbour rows and wall slots in one launch: the rows are read once for the density pass,
+// both solves and XSPH, and the launches between them go. P and A are the divergence solve's, D and B the density solve's
+// (D.vel is P.vel2); `between` are the counters of the barriers between the phases when the liquid outgrew the blocks.
+template <bool MS, bool CG, bool ONE>
+__global__ void __launch_bounds__(SMALL_BLOCK, 1)
+k_small_step(const __grid_constant__ DevP P, const __grid_constant__ DevP D, const __grid_constant__ SolveArgs A,
+             const __grid_constant__ SolveArgs B, int* between) {
+  extern __shared__ float4 small_rows[];
+  if (P.nfw[0] > (int)gridDim.x * SMALL_BLOCK) {
+    constexpr int NBX = 4 | (MS ? MS_FLAG : 0);
+    const int nf = P.nfw[0], all = nf + P.nfw[1], first = blockIdx.x * SMALL_BLOCK + threadIdx.x,
+              step = gridDim.x * SMALL_BLOCK;
+    GridSync sync{0u, gridDim.x + A.extra, between + CT_ARRIVE, A.status, A.wait_limit};
+    for (int p = first; p < nf; p += step) density_one<NBX>(P, p);
+    if (!sync()) return;
+    outgrown_solve<MS, CG, ONE>(P, A);
+    if (!sync()) return;
+    for (int p = first; p < all; p += step) {
+      if (p < nf) xsph_one<NBX>(P, p);
+      else P.vel2[p] = P.vel[p];
+    }
+    if (!sync()) return;
+    outgrown_solve<MS, CG, ONE>(D, B);
+    if (!sync()) return;
+    for (int p = first; p < all; p += step) finish_one<MS>(D, p, nf);
+    return;
+  }
+  SmallSolve<MS, CG, ONE> g{P, A, GridSync{0u, gridDim.x + A.extra, A.ctr + CT_ARRIVE, A.status, A.wait_limit}, small_rows,
+                            reinterpret_cast<int2*>(small_rows + ROW_RES * SMALL_BLOCK)};
+  g.run_step(D, B);
 }
 
 }  // namespace adf
