@@ -220,7 +220,7 @@ struct adf_solver {
   int* perr = nullptr;               // device [1]: a barrier wait gave up
   // the resting-jitter rule (adf_params.jitter_speed > 0): per-world tolerance factor and its float64 sums
   float* jit_scale = nullptr;                 // [W]
-  double *jit_part = nullptr, *jit_flow = nullptr, *jit_head = nullptr;  // [chunks][4], [W][4], [W][4]
+  double* jit_part = nullptr;                 // [chunks][JIT_TERMS]
   __nv_bfloat16 *mw1 = nullptr, *mw2 = nullptr;
   float *mparams = nullptr, *mnorm = nullptr;
   int* merr = nullptr;
@@ -464,18 +464,26 @@ void set_solve_params(adf_solver* s, DevP& P, int mode, double dt) {
   P.relief = (mode == 1 && p.relief_speed > 0.0) ? (float)(p.relief_speed * dt * p.lattice_grad) : (float)(1.0e30);
 }
 
-int prepare(adf_solver* s, DevP& P, cudaStream_t st, bool density = true) {
+// What a step adds to the sort: the state to copy (null where its output array is its input array), and whether the density
+// pass is left to k_small_step.
+struct StepStart {
+  const float *q_in = nullptr, *qd_in = nullptr;
+  bool density = true;
+};
+
+int prepare(adf_solver* s, DevP& P, cudaStream_t st, const StepStart* step = nullptr) {
   const int n = s->n;
   prof_begin(s, 0, st);
   if (P.skin_on) {  // which worlds rebuild their superset rows (dfsph_skin.cuh)
     LAUNCH(s, k_skin_seed, blocks(std::max(s->W, 1)), BLOCK, st, P);
     LAUNCH(s, k_skin_check, blocks(n), BLOCK, st, P);
   }
-  LAUNCH(s, k_classify, blocks(n), BLOCK, st, P);
+  LAUNCH(s, k_classify, blocks(n), BLOCK, st, P, step ? step->q_in : nullptr, step ? step->qd_in : nullptr);
   LAUNCH(s, k_scan_tiles, s->n_tiles, SCAN_THREADS, st, P.counts, s->n_keys, s->tile_sums);
   LAUNCH(s, k_scan_tile_sums, 1, SCAN_THREADS, st, s->tile_sums, s->n_tiles);
   LAUNCH(s, k_scan_apply, s->n_tiles, SCAN_THREADS, st, P.counts, s->n_keys, s->tile_sums, P.cell_start);
-  LAUNCH(s, k_post_scan, blocks(std::max(s->W, 1)), BLOCK, st, P, s->world_cells);
+  LAUNCH(s, k_post_scan, blocks(std::max(s->W, 1)), BLOCK, st, P, s->world_cells, step ? P.max_speed_bits : nullptr,
+         s->solve_ctr, s->solve_ctr ? 3 * CT_SIZE : 0);
   LAUNCH(s, k_scatter, blocks(n), BLOCK, st, P);
   prof_end(s, st);
   prof_begin(s, 1, st);
@@ -501,7 +509,7 @@ int prepare(adf_solver* s, DevP& P, cudaStream_t st, bool density = true) {
   else LAUNCH(s, k_wall_slots<BLOCK>, blocks(n), BLOCK, st, P);
   if (P.slot_cap > 1) LAUNCH(s, k_shape_slots, blocks(n), BLOCK, st, P);
   prof_end(s, st);
-  if (!density) {
+  if (step && !step->density) {
     s->built = true;
     return check_launch();
   }
@@ -676,8 +684,7 @@ int launch_resident(adf_solver* s, const void* kernel, void** args, cudaStream_t
 
 // One solve (or, with init 0, its iterations and apply) in one launch.
 int grid_solve(adf_solver* s, const DevP& P, int mode, int init, cudaStream_t st) {
-  SolveArgs A = solve_args(s, mode, init);
-  CK(cudaMemsetAsync(A.ctr, 0, sizeof(int) * CT_SIZE, st));
+  SolveArgs A = solve_args(s, mode, init);  // counters zeroed by k_post_scan
   void* args[] = {const_cast<DevP*>(&P), &A};
   return launch_resident(s, grid_kernel(s), args, st);
 }
@@ -847,20 +854,15 @@ mlp::Net solver_net(const adf_solver* s) {
   return mlp::Net{s->mw1, s->mw2, s->mparams, s->mnorm, s->merr, mlp::WAIT_LIMIT};
 }
 
-// This step's density tolerance per world (solve_driver.py:99-110), from the last step's density warm starts.
-int density_tolerance(adf_solver* s, DevP& P, double dt, cudaStream_t st) {
-  const int W = s->W;
-  if (P.n_chunks > 0) {
-    LAUNCH(s, k_jitter_chunks, (P.n_chunks + 7) / 8, 256, st, P, 1, s->jit_part);
-    LAUNCH(s, k_jitter_worlds, (W + 7) / 8, 256, st, P, 1, (const double*)s->jit_part, s->jit_head);
-  } else {
-    CK(cudaMemsetAsync(s->jit_head, 0, sizeof(double) * JIT_TERMS * W, st));
-  }
+// This step's density tolerance per world (solve_driver.py:99-110), from the liquid's velocities at its start and the last
+// step's density warm starts.
+void density_tolerance(adf_solver* s, DevP& P, double dt, cudaStream_t st) {
+  if (P.n_chunks > 0)
+    LAUNCH(s, k_jitter_chunks, (P.n_chunks + JIT_WARPS - 1) / JIT_WARPS, 32 * JIT_WARPS, st, P, s->jit_part);
   const adf_params& p = s->prm;
-  LAUNCH(s, k_tol_scale, blocks(W), BLOCK, st, P, (const double*)s->jit_head,
-         p.jitter_ratio > 0.0 ? (const double*)s->jit_flow : nullptr, (float)dt, (float)p.jitter_speed,
-         (float)p.jitter_ratio, (float)p.tol_den, (float)p.tol_den_min, s->jit_scale, s->den_tol);
-  return ADF_OK;
+  LAUNCH(s, k_jitter_worlds, (s->W + JIT_WARPS - 1) / JIT_WARPS, 32 * JIT_WARPS, st, P, (const double*)s->jit_part,
+         p.jitter_ratio > 0.0 ? 1 : 0, (float)dt, (float)p.jitter_speed, (float)p.jitter_ratio, (float)p.tol_den,
+         (float)p.tol_den_min, s->jit_scale, s->den_tol);
 }
 
 // pressure.py:355-390 + solve_driver.py:121-186 (Jacobi branch) + pressure.py:393-480
@@ -882,10 +884,6 @@ int solve(adf_solver* s, DevP& P, int mode, double dt, cudaStream_t st, bool gra
   const bool subset = warm && first && s->judge && !s->cg && !s->feat_rec;
   P.warm_need = subset ? s->warm_need : nullptr;
   if (subset) LAUNCH(s, k_warm_need, blocks(W), BLOCK, st, P, s->warm_need);
-  if (mode == 1 && s->jit_scale && W > 0) {
-    rc = density_tolerance(s, P, dt, st);
-    if (rc) return rc;
-  }
   if (whole) return grid_solve(s, P, mode, 1, st);
   prof_begin(s, 4, st);
   run_tk(s, TK_SOLVE_INIT, st, P);
@@ -1255,8 +1253,6 @@ int adf_create(const adf_params* params, const adf_model* m, int device, adf_sol
   if (p.jitter_speed > 0.0) {
     rc |= s->alloc(&s->jit_scale, W);
     rc |= s->alloc(&s->jit_part, JIT_TERMS * std::max<size_t>(cb.size(), 1));
-    rc |= s->alloc(&s->jit_flow, JIT_TERMS * (size_t)W);
-    rc |= s->alloc(&s->jit_head, JIT_TERMS * (size_t)W);
   }
   rc |= s->alloc(&d.emax, W);
   rc |= s->alloc(&s->iters_den, W);
@@ -1393,7 +1389,6 @@ int adf_create(const adf_params* params, const adf_model* m, int device, adf_sol
   if (s->jit_scale) {
     const std::vector<float> one(W, 1.0f);
     CKC(cudaMemcpy(s->jit_scale, one.data(), sizeof(float) * W, cudaMemcpyHostToDevice));
-    CKC(cudaMemset(s->jit_flow, 0, sizeof(double) * JIT_TERMS * W));
   }
   if (s->n > 0) {
     k_wall_volume<<<blocks(s->n), BLOCK>>>(s->n, m->flags, m->radius, wall_vol);
@@ -1483,9 +1478,6 @@ namespace {
 // One step's work enqueued on `st`; with `graph` the stream is capturing and the solves become WHILE nodes.
 int enqueue_step(adf_solver* s, const float* q_in, const float* qd_in, float* q_out, float* qd_out,
                  const float* f_ext, double dt, cudaStream_t st, bool graph) {
-  const size_t bytes = sizeof(float) * 3 * (size_t)s->n;
-  if (q_out != q_in) CK(cudaMemcpyAsync(q_out, q_in, bytes, cudaMemcpyDeviceToDevice, st));
-  if (qd_out != qd_in) CK(cudaMemcpyAsync(qd_out, qd_in, bytes, cudaMemcpyDeviceToDevice, st));
   DevP P = s->d;
   P.q = q_out;
   P.qd = qd_out;
@@ -1493,19 +1485,27 @@ int enqueue_step(adf_solver* s, const float* q_in, const float* qd_in, float* q_
   P.dt = (float)dt;
   P.n_sinks = (int)s->sinks_h.size();
   P.sinks = s->sinks_d;
-  CK(cudaMemsetAsync(P.max_speed_bits, 0, sizeof(int) * std::max(s->W, 1), st));
-  const bool one = step_in_one(s, P);
-  int rc = prepare(s, P, st, !one);
-  if (rc) return rc;
-  if (s->jit_scale && s->prm.jitter_ratio > 0.0 && P.n_chunks > 0) {  // the liquid's mean start velocity per world
-    LAUNCH(s, k_jitter_chunks, (P.n_chunks + 7) / 8, 256, st, P, 0, s->jit_part);
-    LAUNCH(s, k_jitter_worlds, (s->W + 7) / 8, 256, st, P, 0, (const double*)s->jit_part, s->jit_flow);
+  StepStart start;
+  start.density = !step_in_one(s, P);
+  const size_t bytes = sizeof(float) * 3 * (size_t)s->n;
+  auto meet = [bytes](const float* a, const float* b) {  // two state arrays that share part of their memory
+    const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+    return x < y + bytes && y < x + bytes;
+  };
+  // Two copies of their own where k_skin_check reads the positions before the sort, and where one array's copy would
+  // change what the other's still has to read; else k_classify copies.
+  if (P.skin_on || (q_out != q_in && (meet(q_out, q_in) || meet(q_out, qd_in))) ||
+      (qd_out != qd_in && (meet(qd_out, qd_in) || meet(qd_out, q_in)))) {
+    if (q_out != q_in) CK(cudaMemcpyAsync(q_out, q_in, bytes, cudaMemcpyDeviceToDevice, st));
+    if (qd_out != qd_in) CK(cudaMemcpyAsync(qd_out, qd_in, bytes, cudaMemcpyDeviceToDevice, st));
+  } else {
+    if (q_out != q_in) start.q_in = q_in;
+    if (qd_out != qd_in) start.qd_in = qd_in;
   }
-  if (one) {
-    if (s->jit_scale) {
-      rc = density_tolerance(s, P, dt, st);
-      if (rc) return rc;
-    }
+  int rc = prepare(s, P, st, &start);
+  if (rc) return rc;
+  if (s->jit_scale && s->W > 0) density_tolerance(s, P, dt, st);
+  if (!start.density) {  // one launch for the rest
     set_solve_params(s, P, 0, dt);
     P.feat_on = 0;
     DevP D = P;
@@ -1513,7 +1513,6 @@ int enqueue_step(adf_solver* s, const float* q_in, const float* qd_in, float* q_
     set_solve_params(s, D, 1, dt);
     SolveArgs A = solve_args(s, 0, 1), B = solve_args(s, 1, 1);
     int* between = s->solve_ctr + 2 * CT_SIZE;
-    CK(cudaMemsetAsync(s->solve_ctr, 0, sizeof(int) * 3 * CT_SIZE, st));
     void* args[] = {&P, &D, &A, &B, &between};
     rc = launch_resident(s, small_step_kernel(s), args, st);
     if (rc) return rc;

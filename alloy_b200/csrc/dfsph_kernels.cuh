@@ -275,10 +275,23 @@ __device__ __forceinline__ void cell_coords(const WorldGrid& g, float x, float y
 
 // ------------------------------------------------------------------------------------------------ sorting
 // Groups (neighbors.py:36-51): fluid = ACTIVE and phase >= 1; wall = a boundary particle (PROXY at creation),
-// ACTIVE, in a world; every other particle stays out of the sorted arrays.
-__global__ void k_classify(DevP P) {
+// ACTIVE, in a world; every other particle stays out of the sorted arrays. A step whose output arrays are not its input
+// arrays has the state copied on the way (q_in, qd_in not null).
+__global__ void k_classify(DevP P, const float* q_in, const float* qd_in) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= P.n) return;
+  const float* q = q_in ? q_in : P.q;
+  const float x = q[3 * i], y = q[3 * i + 1], z = q[3 * i + 2];
+  if (q_in) {
+    P.q[3 * i] = x;
+    P.q[3 * i + 1] = y;
+    P.q[3 * i + 2] = z;
+  }
+  if (qd_in) {
+    P.qd[3 * i] = qd_in[3 * i];
+    P.qd[3 * i + 1] = qd_in[3 * i + 1];
+    P.qd[3 * i + 2] = qd_in[3 * i + 2];
+  }
   int w = P.world[i];
   int cls = -1;
   if (w >= 0 && w < P.W) {
@@ -291,7 +304,7 @@ __global__ void k_classify(DevP P) {
   }
   const WorldGrid g = P.grid[w];
   int cx, cy, cz;
-  cell_coords(g, P.q[3 * i], P.q[3 * i + 1], P.q[3 * i + 2], cx, cy, cz);
+  cell_coords(g, x, y, z, cx, cy, cz);
   int key = cls * P.total_cells + cell_key(g, cx, cy, cz);
   P.key_of[i] = key;
   atomicAdd(&P.counts[key], 1);
@@ -378,9 +391,12 @@ __global__ void k_scan_apply(const int* in, int n, const int* tile_off, int* out
   }
 }
 
-// Fluid and wall counts, and each world's liquid count (n_active, an exact integer in float64).
-__global__ void k_post_scan(DevP P, const int* world_cells) {
+// Fluid and wall counts, and each world's liquid count (n_active, an exact integer in float64). In a step also the words
+// it starts from zero: the worlds' largest speeds and the counters of its solves (a memset node each before).
+__global__ void k_post_scan(DevP P, const int* world_cells, int* speed, int* ctr, int ctrs) {
   int w = blockIdx.x * blockDim.x + threadIdx.x;
+  for (int k = w; k < ctrs; k += gridDim.x * blockDim.x) ctr[k] = 0;
+  if (speed && w < P.W) speed[w] = 0;
   if (w == 0) {
     int nf = P.cell_start[P.total_cells];
     P.nfw[0] = nf;
@@ -2828,69 +2844,85 @@ __device__ __forceinline__ float warp_max(float v) {
 // (S1 = sum kd+, S2 = sum kd+^2 over the world's liquid, kd+ = max(kd, 0)) and v = max(speed, ratio |U|), U the mean
 // velocity of the liquid in the step's start state. The sums are float64 over the caller's order in the tree order of
 // the other per-world sums (chunks of 256 by one warp each, then each world's chunks).
-constexpr int JIT_TERMS = 4;
+//
+// Both sums are of the step's start (the warm starts change only with its end), so one pass takes all six terms, a chunk's
+// values loaded once and its six trees side by side: what bounds it is latency (118 warps at 30k particles). Term after term
+// in four launches and a fifth for the factor took 56 us of the 30k tank's step (cold); four steps there with the state
+// copied and the counters cleared in the sort's kernels too: 1,740 -> 1,658 us.
+constexpr int JIT_TERMS = 6;
 
-// term k of particle i (caller's order), 0 unless liquid: flow (k: v_z, 1, v_x, v_y; solve_driver.py:40-51, the
-// step's start velocity) or head (k: kd+, kd+ kd+; solve_driver.py:27-37)
-__device__ __forceinline__ float jitter_term(const DevP& P, int i, int head, int k) {
-  if (!is_fluid_orig(P, i)) return 0.0f;
-  if (!head) {
-    const float* v = P.qd + 3 * (size_t)i;
-    return k == 0 ? v[2] : k == 1 ? 1.0f : k == 2 ? v[0] : v[1];
-  }
+// The terms of particle i (caller's order), 0 unless liquid: flow (v_z, 1, v_x, v_y; solve_driver.py:40-51) and head
+// (kd+, kd+ kd+; solve_driver.py:27-37).
+__device__ __forceinline__ void jitter_terms(const DevP& P, int i, double (&t)[JIT_TERMS]) {
+#pragma unroll
+  for (int k = 0; k < JIT_TERMS; ++k) t[k] = 0.0;
+  if (!is_fluid_orig(P, i)) return;
+  const float* v = P.qd + 3 * (size_t)i;
   const float kd = maxr(P.kd[i], 0.0f);
-  return k == 0 ? kd : kd * kd;
+  t[0] = (double)v[2];
+  t[1] = 1.0;
+  t[2] = (double)v[0];
+  t[3] = (double)v[1];
+  t[4] = (double)kd;
+  t[5] = (double)(kd * kd);
 }
 
-// per chunk (one warp each, 8 per block): the float64 sums of the terms (2 for head, 4 for flow) into part[c][k]
-__global__ void __launch_bounds__(256) k_jitter_chunks(DevP P, int head, double* part) {
-  const int lane = threadIdx.x & 31;
-  const int c = blockIdx.x * 8 + (threadIdx.x >> 5);
+// fold256_warp for JIT_TERMS sums at once: value(L, t) gives value L of each; the sums in lane 0.
+template <class F>
+__device__ __forceinline__ void fold256_jitter(F value, double (&sum)[JIT_TERMS]) {
+  double s[8][JIT_TERMS];
+#pragma unroll
+  for (int g = 0; g < 8; ++g) value(32 * g + (int)(threadIdx.x & 31), s[g]);
+#pragma unroll
+  for (int g = 0; g < 8; ++g)
+#pragma unroll
+    for (int k = 0; k < JIT_TERMS; ++k)
+#pragma unroll
+      for (int o = 16; o >= 1; o >>= 1) s[g][k] = s[g][k] + __shfl_down_sync(0xffffffffu, s[g][k], o);
+#pragma unroll
+  for (int k = 0; k < JIT_TERMS; ++k) {
+#pragma unroll
+    for (int o = 4; o >= 1; o >>= 1)
+#pragma unroll
+      for (int l = 0; l < o; ++l) s[l][k] = s[l][k] + s[l + o][k];
+    sum[k] = s[0][k];
+  }
+}
+
+// per chunk (one warp each): the float64 sums of the terms into part[c][k]
+constexpr int JIT_WARPS = 4;
+
+__global__ void __launch_bounds__(32 * JIT_WARPS) k_jitter_chunks(DevP P, double* part) {
+  const int c = blockIdx.x * JIT_WARPS + (threadIdx.x >> 5);
   if (c >= P.n_chunks) return;
   const int b = P.chunk_begin[c], e = P.chunk_end[c];
-  const int K = head ? 2 : JIT_TERMS;
-  for (int k = 0; k < K; ++k) {
-    const double sum = fold256_warp([&](int L) -> double {
-      const int i = b + L;
-      return i < e ? (double)jitter_term(P, i, head, k) : 0.0;
-    });
-    if (lane == 0) part[(size_t)c * JIT_TERMS + k] = sum;
-  }
+  double sum[JIT_TERMS];
+  fold256_jitter([&](int L, double (&t)[JIT_TERMS]) {
+    if (b + L < e) jitter_terms(P, b + L, t);
+    else
+#pragma unroll
+      for (int k = 0; k < JIT_TERMS; ++k) t[k] = 0.0;
+  }, sum);
+  if ((threadIdx.x & 31) == 0)
+#pragma unroll
+    for (int k = 0; k < JIT_TERMS; ++k) part[(size_t)c * JIT_TERMS + k] = sum[k];
 }
 
-// per world (one warp each): its chunks' partials folded into out[w][k]
-__global__ void __launch_bounds__(256) k_jitter_worlds(DevP P, int head, const double* part, double* out) {
-  const int lane = threadIdx.x & 31;
-  const int w = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (w >= P.W) return;
-  const int c0 = P.world_chunk_start[w], c1 = P.world_chunk_start[w + 1];
-  const int K = head ? 2 : JIT_TERMS;
-  for (int k = 0; k < K; ++k) {
-    const double sum = fold256_warp([&](int L) -> double {
-      double a = 0.0;
-      for (int c = c0 + L; c < c1; c += 256) a = a + part[(size_t)c * JIT_TERMS + k];
-      return a;
-    });
-    if (lane == 0) out[(size_t)w * JIT_TERMS + k] = sum;
-  }
-}
-
-// solve_driver.py:54-74 (tol_scale_kernel) and runtime.py:115-116 (the reported tolerance tol x scale); `flow` null
-// when the flow ratio is 0
-__global__ void k_tol_scale(DevP P, const double* head, const double* flow, float dt, float speed, float ratio,
-                            float tol, float tol_min, float* scale, float* den_tol) {
-  const int w = blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= P.W) return;
+// solve_driver.py:54-74 (tol_scale_kernel) and runtime.py:115-116 (the reported tolerance tol x scale) from a world's sums;
+// `flow` false when the flow ratio is 0.
+__device__ __forceinline__ void tolerance_of(const DevP& P, int w, const double (&sum)[JIT_TERMS], bool flow, float dt,
+                                             float speed, float ratio, float tol, float tol_min, float* scale,
+                                             float* den_tol) {
   float s = 1.0f;
   const float gx = P.gravity[3 * w], gy = P.gravity[3 * w + 1], gz = P.gravity[3 * w + 2];
   const float g = __fsqrt_rn(dot_plain(gx, gy, gz, gx, gy, gz));
-  const float s1 = (float)head[(size_t)w * JIT_TERMS], s2 = (float)head[(size_t)w * JIT_TERMS + 1];
+  const float s1 = (float)sum[4], s2 = (float)sum[5];
   float v = speed;
-  if (flow != nullptr) {
-    const double n = flow[(size_t)w * JIT_TERMS + 1];
+  if (flow) {
+    const double n = sum[1];
     if (ratio > 0.0f && n > 0.0) {
-      const float ux = (float)(flow[(size_t)w * JIT_TERMS + 2] / n), uy = (float)(flow[(size_t)w * JIT_TERMS + 3] / n);
-      const float uz = (float)(flow[(size_t)w * JIT_TERMS] / n);
+      const float ux = (float)(sum[2] / n), uy = (float)(sum[3] / n);
+      const float uz = (float)(sum[0] / n);
       v = maxr(v, ratio * __fsqrt_rn(dot_plain(ux, uy, uz, ux, uy, uz)));
     }
   }
@@ -2900,6 +2932,24 @@ __global__ void k_tol_scale(DevP P, const double* head, const double* flow, floa
   }
   scale[w] = s;
   den_tol[w] = tol * s;
+}
+
+// per world (one warp each): its chunks' partials folded, then its tolerance
+__global__ void __launch_bounds__(32 * JIT_WARPS) k_jitter_worlds(DevP P, const double* part, int flow, float dt, float speed,
+                                                                  float ratio, float tol, float tol_min, float* scale,
+                                                                  float* den_tol) {
+  const int w = blockIdx.x * JIT_WARPS + (threadIdx.x >> 5);
+  if (w >= P.W) return;
+  const int c0 = P.world_chunk_start[w], c1 = P.world_chunk_start[w + 1];
+  double sum[JIT_TERMS];
+  fold256_jitter([&](int L, double (&t)[JIT_TERMS]) {
+#pragma unroll
+    for (int k = 0; k < JIT_TERMS; ++k) t[k] = 0.0;
+    for (int c = c0 + L; c < c1; c += 256)
+#pragma unroll
+      for (int k = 0; k < JIT_TERMS; ++k) t[k] = t[k] + part[(size_t)c * JIT_TERMS + k];
+  }, sum);
+  if ((threadIdx.x & 31) == 0) tolerance_of(P, w, sum, flow != 0, dt, speed, ratio, tol, tol_min, scale, den_tol);
 }
 
 // Per-chunk float64 sums (fold256's tree) and maxima of v, one warp per 256-value chunk, 8 chunks per block (a block
