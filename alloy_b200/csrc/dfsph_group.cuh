@@ -202,6 +202,8 @@ struct GridSolve {
 
   __device__ __forceinline__ int tid() const { return blockIdx.x * blockDim.x + threadIdx.x; }
   __device__ __forceinline__ int threads() const { return gridDim.x * blockDim.x; }
+  // This warp's turn at a list of folds: one for each block before a second, since the warps of an SM share its shuffles.
+  __device__ __forceinline__ int turn() const { return (threadIdx.x >> 5) * gridDim.x + blockIdx.x; }
 
   // f(p, w) for the particles of every listed run. Warps take runs in turn, so that an SM's warps work on neighbouring
   // bricks of cells (runs handed out by a counter evened the SMs out, but the phases of a million particles, bound by
@@ -266,7 +268,7 @@ struct GridSolve {
   // The listed worlds' chunk partials: sums of x and y = value(i, x, y) and the maximum of y, per chunk 256 threads.
   template <class F>
   __device__ __forceinline__ void fold_chunks(F value) {
-    for (int k = tid() >> 5; k < n_chunks; k += threads() >> 5) {  // a warp each
+    for (int k = turn(); k < n_chunks; k += threads() >> 5) {  // a warp each
       const int c = ONE ? c0 + k : __ldcg(&A.chunks[cur][k]);
       const int b = ONE ? ib + 256 * k : P.chunk_begin[c];
       fold_chunk(P, c, b, ONE ? min(b + 256, ie) : P.chunk_end[c], value);
@@ -279,7 +281,7 @@ struct GridSolve {
   // Several worlds: f(w, x, y, mx) in lane 0 of the warp that folds world w.
   template <class F>
   __device__ __forceinline__ void fold_worlds(F f) {
-    for (int k = tid() >> 5; k < n_worlds; k += threads() >> 5) {
+    for (int k = turn(); k < n_worlds; k += threads() >> 5) {
       const int w = __ldcg(&A.worlds[cur][k]);
       double x, y;
       float m;

@@ -2812,24 +2812,38 @@ __global__ void __launch_bounds__(256) k_world_sum2(DevP P, int with_max) {
   if (with_max) P.emax[w] = maxr(mx, 0.0f);
 }
 
-// fold256's tree computed by one warp: value L of the 256 (group L / 32, lane L % 32) comes from value(L); each group
-// of 32 folds by the same shuffles (offsets 16..1), then the 8 group sums fold with offsets 4, 2, 1. Valid in lane 0.
+// fold256's tree computed by one warp, lane l holding value 32 g + l in s[g]: each group of 32 folds with offsets 16..1,
+// then the 8 group sums with offsets 4, 2, 1. The result in every lane. Shuffles are what it costs: folding the groups one
+// by one takes 40 of doubles (80 instructions of a pipe that serves a warp every other cycle, so 32 warps of an SM folding
+// two sums each kept it busy for 5 us). Here a lane gives half of the groups it still holds to its partner and takes the
+// partner's share of the other half, the same pairs added: 4 + 2 + 1 + 1 + 1, and 3 for the group sums. With a fold for each
+// SM before a second, four steps of the 30k column took 2,495 -> 2,307 us, of the 30k tank 1,658 -> 1,520.
+__device__ __forceinline__ double fold256_lanes(double (&s)[8]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 16, m = 4; m >= 1; o >>= 1, m >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < m; ++i) {
+      const double give = up ? s[i] : s[i + m], keep = up ? s[i + m] : s[i];
+      s[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  double v = s[0];  // of group lane / 4, in its four lanes
+  v = v + __shfl_xor_sync(0xffffffffu, v, 2);
+  v = v + __shfl_xor_sync(0xffffffffu, v, 1);
+#pragma unroll
+  for (int o = 16; o >= 4; o >>= 1) v = v + __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// fold256_lanes of value(L), L of the 256
 template <class F>
 __device__ __forceinline__ double fold256_warp(F value) {
-  const int lane = threadIdx.x & 31;
   double s[8];
 #pragma unroll
-  for (int g = 0; g < 8; ++g) {
-    double v = value(32 * g + lane);
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) v = v + __shfl_down_sync(0xffffffffu, v, o);
-    s[g] = v;
-  }
-#pragma unroll
-  for (int o = 4; o >= 1; o >>= 1)
-#pragma unroll
-    for (int l = 0; l < o; ++l) s[l] = s[l] + s[l + o];
-  return s[0];
+  for (int g = 0; g < 8; ++g) s[g] = value(32 * g + (int)(threadIdx.x & 31));
+  return fold256_lanes(s);
 }
 
 __device__ __forceinline__ float warp_max(float v) {
@@ -2867,26 +2881,19 @@ __device__ __forceinline__ void jitter_terms(const DevP& P, int i, double (&t)[J
   t[5] = (double)(kd * kd);
 }
 
-// fold256_warp for JIT_TERMS sums at once: value(L, t) gives value L of each; the sums in lane 0.
+// fold256_warp for JIT_TERMS sums at once: value(L, t) gives value L of each.
 template <class F>
 __device__ __forceinline__ void fold256_jitter(F value, double (&sum)[JIT_TERMS]) {
-  double s[8][JIT_TERMS];
+  double s[JIT_TERMS][8];
 #pragma unroll
-  for (int g = 0; g < 8; ++g) value(32 * g + (int)(threadIdx.x & 31), s[g]);
+  for (int g = 0; g < 8; ++g) {
+    double t[JIT_TERMS];
+    value(32 * g + (int)(threadIdx.x & 31), t);
 #pragma unroll
-  for (int g = 0; g < 8; ++g)
-#pragma unroll
-    for (int k = 0; k < JIT_TERMS; ++k)
-#pragma unroll
-      for (int o = 16; o >= 1; o >>= 1) s[g][k] = s[g][k] + __shfl_down_sync(0xffffffffu, s[g][k], o);
-#pragma unroll
-  for (int k = 0; k < JIT_TERMS; ++k) {
-#pragma unroll
-    for (int o = 4; o >= 1; o >>= 1)
-#pragma unroll
-      for (int l = 0; l < o; ++l) s[l][k] = s[l][k] + s[l + o][k];
-    sum[k] = s[0][k];
+    for (int k = 0; k < JIT_TERMS; ++k) s[k][g] = t[k];
   }
+#pragma unroll
+  for (int k = 0; k < JIT_TERMS; ++k) sum[k] = fold256_lanes(s[k]);
 }
 
 // per chunk (one warp each): the float64 sums of the terms into part[c][k]
@@ -3235,26 +3242,9 @@ template <class F>
 __device__ __forceinline__ void fold256_warp2(F value, double& rx, double& ry) {
   double sx[8], sy[8];
 #pragma unroll
-  for (int g = 0; g < 8; ++g) {
-    double x, y;
-    value(32 * g + (threadIdx.x & 31), x, y);
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) {
-      x = x + __shfl_down_sync(0xffffffffu, x, o);
-      y = y + __shfl_down_sync(0xffffffffu, y, o);
-    }
-    sx[g] = x;
-    sy[g] = y;
-  }
-#pragma unroll
-  for (int o = 4; o >= 1; o >>= 1)
-#pragma unroll
-    for (int l = 0; l < o; ++l) {
-      sx[l] = sx[l] + sx[l + o];
-      sy[l] = sy[l] + sy[l + o];
-    }
-  rx = sx[0];
-  ry = sy[0];
+  for (int g = 0; g < 8; ++g) value(32 * g + (int)(threadIdx.x & 31), sx[g], sy[g]);
+  rx = fold256_lanes(sx);
+  ry = fold256_lanes(sy);
 }
 
 // k_sums2_fused with one warp per chunk (8 per block), for models whose worlds have at most WARP_FOLD_MAX_CHUNKS

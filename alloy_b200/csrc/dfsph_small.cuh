@@ -49,7 +49,8 @@ struct SmallSolve {
 
   __device__ __forceinline__ int tid() const { return blockIdx.x * SMALL_BLOCK + threadIdx.x; }
   __device__ __forceinline__ int threads() const { return gridDim.x * SMALL_BLOCK; }
-  __device__ __forceinline__ int warp() const { return tid() >> 5; }
+  // this warp's turn at a list of folds: one for each block before a second (GridSolve::turn)
+  __device__ __forceinline__ int warp() const { return (threadIdx.x >> 5) * gridDim.x + blockIdx.x; }
   __device__ __forceinline__ int warps() const { return threads() >> 5; }
   __device__ __forceinline__ int at(int k) const { return k * SMALL_BLOCK + threadIdx.x; }
 
