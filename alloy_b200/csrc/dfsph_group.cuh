@@ -196,7 +196,8 @@ struct GridSolve {
   GridSync sync;
   int cur;           // the lists of the running iteration, and their lengths
   int n_worlds, n_items, n_chunks;
-  int2 first;        // this warp's first list entry
+  int run0;          // this warp's first list entry
+  int2 first;        // (its value)
   // ONE: the world's liquid range, caller range and chunks
   int lb, le, ib, ie, c0, c1;
 
@@ -215,7 +216,7 @@ struct GridSolve {
     } else {
       const int lane = threadIdx.x & 31, step = threads() / RUN;
       int2 r = first;
-      for (int i = tid() / RUN; i < n_items; i += step) {
+      for (int i = run0; i < n_items; i += step) {
         int2 next = r;
         if (i + step < n_items) next = __ldcg(&A.items[cur][i + step]);
         if (lane < (r.y & 63)) f(r.x + lane, r.y >> 6);
@@ -234,7 +235,15 @@ struct GridSolve {
       n_worlds = (int)(v >> (2 * LIST_BITS));
       n_items = (int)(v >> LIST_BITS) & LIST_MASK;
       n_chunks = (int)v & LIST_MASK;
-      if (tid() / RUN < n_items) first = __ldcg(&A.items[cur][tid() / RUN]);
+      // Its place among them is the warp's own, so that an SM's warps take neighbouring runs; where there are fewer runs
+      // than warps (few worlds still iterate), the blocks take even shares and no SM idles while others work through 32
+      // warps' gathers.
+      run0 = tid() / RUN;
+      if (n_items < threads() / RUN) {
+        const int share = (n_items + (int)gridDim.x - 1) / (int)gridDim.x, wid = threadIdx.x / RUN;
+        run0 = wid < share ? (int)blockIdx.x * share + wid : n_items;
+      }
+      if (run0 < n_items) first = __ldcg(&A.items[cur][run0]);
     }
   }
   __device__ __forceinline__ unsigned long long* lists() const {
