@@ -697,7 +697,13 @@ bool step_in_one(const adf_solver* s, const DevP& P) {
 
 // Shape of the cooperative launch, from the particles that are or can become liquid (`sph`). Up to SMALL_BLOCK of them
 // per SM their rows fit the SMs' shared memory (dfsph_small.cuh). Above, a thread each while the device holds that many:
-// every SM gets an even share. Above that, the form that takes fewer rounds (dfsph_group.cuh).
+// every SM gets an even share. Above that, the form that takes fewer rounds (dfsph_group.cuh), for the Jacobi up to
+// JACOBI_ROUNDS of the deep one: past those a launch per phase, dealt out block by block and tuned to the model, costs less
+// than its boundaries (a step, one launch against one per phase: 3.1M particles 6.16 against 6.40 ms, pour of 1,024 worlds
+// 13.49 against 13.83, 6.3M particles 12.26 against 12.27, batched 512 worlds 12.91 against 12.78, pour of 2,048 worlds 27.2
+// against 26.5, of 4,096 56.8 against 52.7). The CG, whose launches per phase cover converged worlds too, gains at every
+// size (2,048 worlds 33.3 against 37.5).
+constexpr long long JACOBI_ROUNDS = 40;
 int setup_grid_solve(adf_solver* s, int sph) {
   CK(cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, s->device));
   const int sms = s->sms;
@@ -707,6 +713,7 @@ int setup_grid_solve(adf_solver* s, int sph) {
   int greatest = 0;
   CK(cudaDeviceGetStreamPriorityRange(&s->least_priority, &greatest));
   const long long deep = (long long)sms * GRID_BLOCK, wide = 2ll * sms * WIDE_BLOCK, n = std::max(sph, 1);
+  if (!s->cg && n > JACOBI_ROUNDS * deep) return ADF_OK;
   if (n <= (long long)sms * SMALL_BLOCK) {
     s->grid_form = 0;
     s->grid_threads = SMALL_BLOCK;

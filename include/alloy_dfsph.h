@@ -183,7 +183,8 @@ int adf_halo_stats(adf_solver* solver, int32_t* in_use, int64_t* stats, void* st
  * 254-297, inside wp.capture_while, solve_driver.py:186). Each pressure solve, its start, every iteration of every world
  * and the velocity update, runs as ONE cooperative launch whose phases are separated by grid-wide barriers, instead of
  * four graph nodes per Jacobi iteration or ten per CG iteration; the results are the same bits. This is what a new
- * solver does, except in steps that time kernels one by one (tuning, profiling) and with item halos on. enable = 1 does
+ * solver does, except in steps that time kernels one by one (tuning, profiling), with item halos on and for the Jacobi on
+ * some millions of particles, where a kernel per phase is the faster. enable = 1 does
  * it in the tuning step too, for the projected CG; 0 launches one kernel per phase. Every barrier wait is bounded: a
  * wait that gives up sets the solver's status, after which adf_get_report returns ADF_ERR_STATE until
  * adf_clear_status. The launch occupies every SM of the device it finds free and is dispatched at the lowest stream
