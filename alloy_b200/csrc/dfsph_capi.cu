@@ -188,12 +188,13 @@ struct adf_solver {
     const void* key[5];
     double dt;
     unsigned version;
+    bool raised;
+    long long kernels;  // it launches outside its WHILE bodies
     cudaGraphExec_t exec;
   };
   std::vector<GraphEntry> graphs;
   unsigned table_version = 0;
   bool use_graphs = true;
-  long long graph_kernels = 0;  // kernels a step graph launches outside its WHILE bodies
   long long body_kernels = 0;   // kernels of one WHILE-body iteration
   unsigned long long* body_runs = nullptr;  // device [2]: WHILE-body iterations run so far, those of the running loop
   cudaStream_t cap_stream = nullptr, body_stream = nullptr;
@@ -206,7 +207,8 @@ struct adf_solver {
   int sms = 148;             // the device's multiprocessors
   int grid_blocks = 0;       // blocks of the launch (0: none)
   int grid_threads = 0;      // threads of each
-  int least_priority = 0;
+  int least_priority = 0;    // of the device's streams
+  bool raised = false;       // the running call's stream has a higher one (set_stream)
   int grid_form = 0;         // 0 rows in shared memory (dfsph_small.cuh), 1 deep blocks, 2 wide (dfsph_group.cuh)
   int solve_runs = 0;                     // capacity of a list of runs
   int* solve_ctr = nullptr;  // [3][CT_SIZE]: one set per solve of a step, one for the barriers between them
@@ -604,14 +606,26 @@ void cg_iteration(adf_solver* s, DevP& P, cudaStream_t st) {
   LAUNCH(s, k_cg_direction, blocks(n), BLOCK, st, P);
 }
 
-// Whether this solve runs as one cooperative launch (dfsph_group.cuh). Steps that time kernels (tuning, profiling) and
-// staged item halos take the kernels one by one, and so does a solver told to (adf_set_persistent 0). The launch was
+// A call that may solve starts on stream `st`. On a stream of raised priority the solves take a kernel per phase, each at
+// that priority: of two cooperative launches of different priorities the later one could take the SMs that the blocks
+// still missing from the earlier one wait for, with neither wholly resident; of equal ones the first is dispatched whole.
+// (A replayed graph's kernels have the priority of the stream it is launched on, whatever their own attribute says.)
+int set_stream(adf_solver* s, cudaStream_t st) {
+  int priority = 0;
+  CK(cudaStreamGetPriority(st, &priority));
+  s->raised = priority < s->least_priority;  // a higher priority is a lower number
+  return ADF_OK;
+}
+
+// Whether this solve runs as one cooperative launch (dfsph_group.cuh). Steps that time kernels (tuning, profiling), steps
+// on a stream of raised priority and staged item halos take the kernels one by one, and so does a solver told to
+// (adf_set_persistent 0). The launch was
 // the faster one at every size measured, or equal (four steps, one kernel per phase against one launch): 2,016
 // particles 1.26 against 0.84 ms, the 30k column 4.08 against 2.56, 123k 1.89 against 1.55, 250k 3.07 against 2.70, the
 // 1M dam break 9.30 against 8.76, 256 columns 24.1 against 20.9, 6 worlds 1.90 against 1.61, 160 worlds 17.6 against
 // 17.4, the pour's first 1,024 worlds 60.6 against 59.8.
 bool grid_solves(const adf_solver* s, const DevP& P) {
-  if (P.n_chunks == 0 || s->W == 0 || s->prof_on || s->grid_blocks == 0) return false;
+  if (P.n_chunks == 0 || s->W == 0 || s->prof_on || s->grid_blocks == 0 || s->raised) return false;
   if (s->persist == 1 && s->cg) return true;
   return s->persist != 0 && !s->tuning && s->halo_mode == 0;
 }
@@ -668,15 +682,11 @@ int launch_resident(adf_solver* s, const void* kernel, void** args, cudaStream_t
   cfg.blockDim = dim3((unsigned)s->grid_threads);
   cfg.dynamicSmemBytes = s->grid_form == 0 ? SMALL_SMEM : 0;
   cfg.stream = st;
-  cudaLaunchAttribute at[2];
+  cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeCooperative;  // every block resident: the barriers wait on all of them
   at[0].val.cooperative = 1;
-  // one priority whatever the stream's: two solvers' launches on streams of different priorities would otherwise take
-  // SMs from each other with neither wholly resident; of equal ones the first is dispatched whole
-  at[1].id = cudaLaunchAttributePriority;
-  at[1].val.priority = s->least_priority;
   cfg.attrs = at;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = 1;
   CK(cudaLaunchKernelExC(&cfg, kernel, args));
   ++s->launches;
   return ADF_OK;
@@ -1568,9 +1578,9 @@ int graph_step(adf_solver* s, const float* q_in, const float* qd_in, float* q_ou
                double dt, cudaStream_t st) {
   const void* key[5] = {q_in, qd_in, q_out, qd_out, f_ext};
   for (auto& g : s->graphs) {
-    if (g.dt == dt && g.version == s->table_version && std::equal(key, key + 5, g.key)) {
+    if (g.dt == dt && g.version == s->table_version && g.raised == s->raised && std::equal(key, key + 5, g.key)) {
       CK(cudaGraphLaunch(g.exec, st));
-      s->launches += s->graph_kernels;
+      s->launches += g.kernels;
       return ADF_OK;
     }
   }
@@ -1581,7 +1591,7 @@ int graph_step(adf_solver* s, const float* q_in, const float* qd_in, float* q_ou
   int rc = enqueue_step(s, q_in, qd_in, q_out, qd_out, f_ext, dt, s->cap_stream, true);
   cudaGraph_t g = nullptr;
   cudaError_t e = cudaStreamEndCapture(s->cap_stream, &g);
-  s->graph_kernels = s->launches - before;
+  const long long kernels = s->launches - before;
   s->launches = before;
   if (rc || e != cudaSuccess) {
     if (g) cudaGraphDestroy(g);
@@ -1599,10 +1609,12 @@ int graph_step(adf_solver* s, const float* q_in, const float* qd_in, float* q_ou
   std::copy(key, key + 5, ge.key);
   ge.dt = dt;
   ge.version = s->table_version;
+  ge.raised = s->raised;
+  ge.kernels = kernels;
   ge.exec = exec;
   s->graphs.push_back(ge);
   CK(cudaGraphLaunch(exec, st));
-  s->launches += s->graph_kernels;
+  s->launches += kernels;
   return ADF_OK;
 }
 }  // namespace
@@ -1619,6 +1631,8 @@ int adf_step(adf_solver* s, const float* q_in, const float* qd_in, float* q_out,
   CK(cudaSetDevice(s->device));
   cudaStreamCaptureStatus cs;
   CK(cudaStreamIsCapturing(st, &cs));
+  const int rc_stream = set_stream(s, st);
+  if (rc_stream) return rc_stream;
   if (cs == cudaStreamCaptureStatusActive)  // the caller is capturing: the step joins its graph
     return enqueue_step(s, q_in, qd_in, q_out, qd_out, f_ext, dt, st, true);
   if (s->tune_pending) {  // the tuning step: kernels one by one, each tuned kernel timed on this step's inputs
@@ -1805,7 +1819,9 @@ int adf_prime(adf_solver* s, const float* q, const float* qd, double dt, double 
   P.n_sinks = 0;
   P.min_nb = 0.0f;
   P.max_it = max_it;
-  int rc = prepare(s, P, st);
+  int rc = set_stream(s, st);
+  if (rc) return rc;
+  rc = prepare(s, P, st);
   if (rc) return rc;
   run_tk(s, TK_XSPH, st, P);  // the velocity one gravity step adds (no pressure guess yet)
   std::swap(P.vel, P.vel2);

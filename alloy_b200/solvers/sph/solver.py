@@ -438,8 +438,9 @@ class SolverDFSPH:
 
     def persistent(self, enable: bool = True) -> None:
         """Whole pressure solves as one cooperative launch with grid-wide barriers (include/alloy_dfsph.h
-        adf_set_persistent), which a new solver does by itself; False: one kernel per phase. The results are the same
-        bits either way."""
+        adf_set_persistent), which a new solver does by itself; False: one kernel per phase, for a program whose other
+        kernels hold SMs for long or wait for the step's result while they run. A step on a stream of raised priority
+        launches one kernel per phase, at that priority. The results are the same bits either way."""
         _lib.check(self._lib.adf_set_persistent(self._h, int(bool(enable))), "persistent")
 
     def halo(self, mode: int = 1) -> None:

@@ -187,8 +187,14 @@ int adf_halo_stats(adf_solver* solver, int32_t* in_use, int64_t* stats, void* st
  * some millions of particles, where a kernel per phase is the faster. enable = 1 does
  * it in the tuning step too, for the projected CG; 0 launches one kernel per phase. Every barrier wait is bounded: a
  * wait that gives up sets the solver's status, after which adf_get_report returns ADF_ERR_STATE until
- * adf_clear_status. The launch occupies every SM of the device it finds free and is dispatched at the lowest stream
- * priority. */
+ * adf_clear_status.
+ *
+ * Beside other work on the device: all blocks of the launch are resident at once, on models of more than 256 liquid
+ * particles per SM one or two blocks on every SM. A kernel of another stream that holds an SM delays the whole solve until it
+ * ends, where launches per phase went on with the other SMs; a kernel that holds an SM until it sees the solve's result
+ * must not run beside it. Programs with such kernels take 0. A step on a stream of raised priority launches one kernel per
+ * phase, each at that priority, whatever `enable` says (a captured step keeps the form of the stream it was captured
+ * on, and is to be launched on streams of that priority). */
 int adf_set_persistent(adf_solver* solver, int enable);
 /* Test hook of the bounded barrier waits: each wait polls at most `polls` times (default 33,554,432, some twenty
  * seconds),
