@@ -108,6 +108,11 @@ int fail(int code, const std::string& msg) {
 // Packed words of a report: three 8-byte and fifteen 4-byte arrays per world, two status words.
 inline size_t report_words(int W) { return (size_t)W * (3 * 2 + 15) + 2; }
 
+int fail_wait() {
+  return fail(ADF_ERR_STATE, "pressure solve: a grid-barrier wait of the persistent CG solve expired; the step's "
+                             "results are invalid");
+}
+
 inline int blocks(long long n, int b = BLOCK) { return (int)((n + b - 1) / b); }
 
 // Models up to this many particles take the CG products by teams of TL lanes per particle: below it one lane per
@@ -219,7 +224,8 @@ struct adf_solver {
   int halo_items = 0;  // item numbers k_halo covers: n / 256 + W + 1
   unsigned persist_extra = 0;        // extra arrivals a barrier waits for (only the wait-expiry test sets it)
   long long persist_wait = 1 << 25;  // polls of one barrier wait (some twenty seconds) before it gives up
-  int* perr = nullptr;               // device [1]: a barrier wait gave up
+  int* perr = nullptr;               // device [4]: a barrier wait gave up; the address of perr_host (8 bytes)
+  int* perr_host = nullptr;          // pinned [1]: as perr, for the calls that do not synchronise
   // the resting-jitter rule (adf_params.jitter_speed > 0): per-world tolerance factor and its float64 sums
   float* jit_scale = nullptr;                 // [W]
   double* jit_part = nullptr;                 // [chunks][JIT_TERMS]
@@ -605,6 +611,10 @@ void cg_iteration(adf_solver* s, DevP& P, cudaStream_t st) {
   }
   LAUNCH(s, k_cg_direction, blocks(n), BLOCK, st, P);
 }
+
+// Whether a solve's barrier wait has given up since the last adf_clear_status, as far as the host can know without waiting
+// for the device: the state and the warm starts that the next step would go on from are invalid.
+bool wait_failed(const adf_solver* s) { return *(volatile const int*)s->perr_host != 0; }
 
 // A call that may solve starts on stream `st`. On a stream of raised priority the solves take a kernel per phase, each at
 // that priority: of two cooperative launches of different priorities the later one could take the SMs that the blocks
@@ -1439,8 +1449,11 @@ int adf_create(const adf_params* params, const adf_model* m, int device, adf_sol
   CKC(cudaStreamCreateWithFlags(&s->body_stream, cudaStreamNonBlocking));
   CKC(cudaMalloc(&s->body_runs, 2 * sizeof(unsigned long long)));
   CKC(cudaMemset(s->body_runs, 0, 2 * sizeof(unsigned long long)));
-  CKC(cudaMalloc(&s->perr, sizeof(int)));
-  CKC(cudaMemset(s->perr, 0, sizeof(int)));
+  CKC(cudaMalloc(&s->perr, 4 * sizeof(int)));
+  CKC(cudaMemset(s->perr, 0, 4 * sizeof(int)));
+  CKC(cudaHostAlloc((void**)&s->perr_host, sizeof(int), cudaHostAllocDefault));
+  *s->perr_host = 0;
+  CKC(cudaMemcpy(s->perr + 2, &s->perr_host, sizeof(int*), cudaMemcpyHostToDevice));
   CKC(cudaEventCreate(&s->tev[0]));
   CKC(cudaEventCreate(&s->tev[1]));
   CKC(cudaMalloc(&s->snap_kappa, sizeof(float) * n));
@@ -1475,6 +1488,7 @@ void adf_destroy(adf_solver* s) {
   if (s->list_entries) cudaFree(s->list_entries);
   if (s->body_runs) cudaFree(s->body_runs);
   if (s->perr) cudaFree(s->perr);
+  if (s->perr_host) cudaFreeHost(s->perr_host);
   for (auto& g : s->graphs) cudaGraphExecDestroy(g.exec);
   if (s->cap_stream) cudaStreamDestroy(s->cap_stream);
   if (s->body_stream) cudaStreamDestroy(s->body_stream);
@@ -1627,6 +1641,7 @@ int adf_step(adf_solver* s, const float* q_in, const float* qd_in, float* q_out,
   if (!(dt > 0.0)) return fail(ADF_ERR_VALUE, "SolverDFSPH.step: dt must be > 0, got " + std::to_string(dt));
   if (s->n == 0) return ADF_OK;
   if (!q_in || !qd_in || !q_out || !qd_out) return fail(ADF_ERR_VALUE, "adf_step: null state array");
+  if (wait_failed(s)) return fail_wait();
   cudaStream_t st = (cudaStream_t)stream;
   CK(cudaSetDevice(s->device));
   cudaStreamCaptureStatus cs;
@@ -1657,6 +1672,7 @@ int adf_density_ratio(adf_solver* s, const float* q, const float* qd, float* rat
                       void* stream) {
   if (!s || !q || !qd) return fail(ADF_ERR_VALUE, "adf_density_ratio: null argument");
   if (s->n == 0) return ADF_OK;
+  if (wait_failed(s)) return fail_wait();
   cudaStream_t st = (cudaStream_t)stream;
   CK(cudaSetDevice(s->device));
   DevP P = s->d;
@@ -1726,9 +1742,7 @@ int adf_get_report(adf_solver* s, adf_report* r, void* stream) {
   for (const Field& f : all)
     if (f.dst && f.src) std::memcpy(f.dst, s->report_host + R.offset[fields++], f.bytes);
   if (merr) return fail(ADF_ERR_STATE, "warm-start network: a tensor-core wait expired; the learned starts are invalid");
-  if (perr)
-    return fail(ADF_ERR_STATE, "pressure solve: a grid-barrier wait of the persistent CG solve expired; the step's "
-                               "results are invalid");
+  if (perr) return fail_wait();
   return ADF_OK;
 }
 
@@ -1809,6 +1823,7 @@ int adf_prime(adf_solver* s, const float* q, const float* qd, double dt, double 
   if (!(dt > 0.0) || !(tol > 0.0) || max_it < 1) return fail(ADF_ERR_VALUE, "adf_prime: dt, tol and max_it must be > 0");
   if (iters) *iters = 0;
   if (s->n == 0) return ADF_OK;
+  if (wait_failed(s)) return fail_wait();
   cudaStream_t st = (cudaStream_t)stream;
   CK(cudaSetDevice(s->device));
   DevP P = s->d;
@@ -1845,6 +1860,7 @@ int adf_prime(adf_solver* s, const float* q, const float* qd, double dt, double 
     std::vector<int> it(std::max(s->W, 1), 0);
     CK(cudaMemcpyAsync(it.data(), s->iters_div, sizeof(int) * s->W, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    if (wait_failed(s)) return fail_wait();
     for (int w = 0; w < s->W; ++w) *iters = std::max(*iters, it[w]);
   }
   return ADF_OK;
@@ -1966,6 +1982,7 @@ int adf_clear_status(adf_solver* s) {
   CK(cudaSetDevice(s->device));
   CK(cudaDeviceSynchronize());
   CK(cudaMemset(s->perr, 0, sizeof(int)));
+  *s->perr_host = 0;
   if (s->merr) CK(cudaMemset(s->merr, 0, sizeof(int)));
   // a launch that left at a barrier may have left the reductions' tickets counted part way
   CK(cudaMemset(s->d.wdone, 0, sizeof(int) * std::max(s->W, 1)));

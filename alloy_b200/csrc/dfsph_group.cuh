@@ -43,7 +43,7 @@ struct SolveArgs {
   int* worlds[2];
   unsigned extra;        // extra arrivals a barrier waits for (only the wait-expiry test sets it)
   long long wait_limit;  // polls of one wait before it gives up
-  int* status;           // set to 1 when a wait gave up
+  int* status;           // set to 1 when a wait gave up; [2], 8 bytes: the host word that is set with it
   int* iters_out;        // [W] the solve's statistics
   float* mean_out;
   float* max_out;        // null: not kept (divergence)
@@ -73,6 +73,7 @@ struct GridSync {
         }
         if (it >= wait_limit) {
           atomicExch(status, 1);
+          *reinterpret_cast<int* volatile*>(status + 2)[0] = 1;  // the host's next call sees it without a read-back
           bad = 1;
           break;
         }

@@ -187,7 +187,8 @@ int adf_halo_stats(adf_solver* solver, int32_t* in_use, int64_t* stats, void* st
  * some millions of particles, where a kernel per phase is the faster. enable = 1 does
  * it in the tuning step too, for the projected CG; 0 launches one kernel per phase. Every barrier wait is bounded: a
  * wait that gives up sets the solver's status, after which adf_get_report returns ADF_ERR_STATE until
- * adf_clear_status.
+ * adf_clear_status, and so do adf_step, adf_density_ratio and adf_prime, which do not synchronise, once the host has seen
+ * it (at the latest when a synchronisation has followed the failed launch).
  *
  * Beside other work on the device: all blocks of the launch are resident at once, on models of more than 256 liquid
  * particles per SM one or two blocks on every SM. A kernel of another stream that holds an SM delays the whole solve until it
