@@ -223,7 +223,7 @@ struct adf_solver {
   int halo_mode = 0;
   int halo_items = 0;  // item numbers k_halo covers: n / 256 + W + 1
   unsigned persist_extra = 0;        // extra arrivals a barrier waits for (only the wait-expiry test sets it)
-  long long persist_wait = 1 << 25;  // polls of one barrier wait (some twenty seconds) before it gives up
+  long long persist_wait = ADF_BARRIER_POLLS;  // of one barrier wait before it gives up
   int* perr = nullptr;               // device [4]: a barrier wait gave up; the address of perr_host (8 bytes)
   int* perr_host = nullptr;          // pinned [1]: as perr, for the calls that do not synchronise
   // the resting-jitter rule (adf_params.jitter_speed > 0): per-world tolerance factor and its float64 sums

@@ -458,9 +458,10 @@ class SolverDFSPH:
         return {"accel": bool(use[0]), "jacobi": bool(use[1]), "staged": int(st[0]), "global": int(st[1]),
                 "records": int(st[2]), "max_records": int(st[3])}
 
-    def barrier_wait(self, polls: int = 1 << 22, extra_arrivals: int = 0) -> None:
-        """Test hook of the persistent solve's bounded barrier waits (adf_set_barrier_wait): polls per wait, and
-        arrivals a barrier waits for beyond the grid's blocks (nonzero makes every wait run out)."""
+    def barrier_wait(self, polls: int = _lib.ADF_BARRIER_POLLS, extra_arrivals: int = 0) -> None:
+        """Test hook of the one-launch solves' bounded barrier waits (adf_set_barrier_wait): polls per wait, and
+        arrivals a barrier waits for beyond the grid's blocks (nonzero makes every wait run out). Without arguments: the
+        library's defaults."""
         _lib.check(self._lib.adf_set_barrier_wait(self._h, int(polls), int(extra_arrivals)), "barrier_wait")
 
     def clear_status(self) -> None:

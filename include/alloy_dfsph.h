@@ -197,10 +197,11 @@ int adf_halo_stats(adf_solver* solver, int32_t* in_use, int64_t* stats, void* st
  * phase, each at that priority, whatever `enable` says (a captured step keeps the form of the stream it was captured
  * on, and is to be launched on streams of that priority). */
 int adf_set_persistent(adf_solver* solver, int enable);
-/* Test hook of the bounded barrier waits: each wait polls at most `polls` times (default 33,554,432, some twenty
- * seconds),
- * and a barrier waits for `extra_arrivals` more blocks than the grid has (default 0; any other value makes every wait
- * run out, which is what the wait-expiry test checks). */
+/* Test hook of the bounded barrier waits: each wait polls at most `polls` times (ADF_BARRIER_POLLS by default, some
+ * twenty seconds: long enough for blocks that have started to wait for the others behind another stream's kernels), and a
+ * barrier waits for `extra_arrivals` more blocks than the grid has (default 0; any other value makes every wait run out,
+ * which is what the wait-expiry tests check). */
+#define ADF_BARRIER_POLLS (1ll << 25)
 int adf_set_barrier_wait(adf_solver* solver, long long polls, int extra_arrivals);
 /* Clears the status words of the bounded waits (the solves' grid barriers and the warm-start network's
  * tensor-core waits) and the per-world reduction tickets a launch that gave up may have left counted, after
