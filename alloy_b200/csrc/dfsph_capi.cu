@@ -109,8 +109,8 @@ int fail(int code, const std::string& msg) {
 inline size_t report_words(int W) { return (size_t)W * (3 * 2 + 15) + 2; }
 
 int fail_wait() {
-  return fail(ADF_ERR_STATE, "pressure solve: a grid-barrier wait of the persistent CG solve expired; the step's "
-                             "results are invalid");
+  return fail(ADF_ERR_STATE, "pressure solve: a grid-barrier wait of a solve in one launch expired; the results since are "
+                             "invalid");
 }
 
 inline int blocks(long long n, int b = BLOCK) { return (int)((n + b - 1) / b); }

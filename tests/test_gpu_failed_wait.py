@@ -102,3 +102,14 @@ def test_a_priming_that_fails_says_so(cuda):
     sol.barrier_wait()
     sol.prime(sc.model.state(), sc.dt)
     sol.report()
+
+
+@pytest.mark.parametrize("solver", ["jacobi", "cg"])
+def test_the_message_names_the_launch_that_failed(cuda, solver):
+    sc = _scene(cuda, (8, 8, 10), 1, solver)
+    sol = _solver(sc)
+    a, b = sc.model.state(), sc.model.state()
+    sol.barrier_wait(polls=2000, extra_arrivals=1)
+    sol.step(a, b, None, None, sc.dt)
+    with pytest.raises(RuntimeError, match="grid-barrier wait of a solve in one launch"):
+        sol.report()
