@@ -33,7 +33,9 @@ constexpr int RUN = 32;                             // particles of a list entry
 // one 64-bit word (worlds << 44 | items << 22 | chunks) that a world joins with one atomic.
 constexpr int CT_ARRIVE = 0, CT_LISTS = 32, CT_CLAMPED = 36, CT_SIZE = 64;
 constexpr int LIST_BITS = 22, LIST_MASK = (1 << LIST_BITS) - 1;
-constexpr long long LIST_MAX_WORLDS = 1 << 20, LIST_MAX_ITEMS = LIST_MASK;
+constexpr long long LIST_MAX_WORLDS = (1 << (64 - 2 * LIST_BITS)) - 1, LIST_MAX_ITEMS = LIST_MASK;
+static_assert(LIST_MAX_WORLDS >> (64 - 2 * LIST_BITS) == 0 && LIST_MAX_ITEMS >> LIST_BITS == 0,
+              "the largest counts fit their fields of the word");
 
 struct SolveArgs {
   int init;              // 1: the start (source, bounds, warm start) is part of this launch; 0: it ran before
