@@ -1968,6 +1968,14 @@ int adf_set_persistent(adf_solver* s, int enable) {
   return ADF_OK;
 }
 
+int adf_solve_launch(const adf_solver* s, int32_t* shape) {
+  if (!s || !shape) return fail(ADF_ERR_VALUE, "adf_solve_launch: null argument");
+  shape[0] = s->grid_blocks > 0 ? s->grid_form : -1;
+  shape[1] = s->grid_blocks;
+  shape[2] = s->grid_blocks > 0 ? s->grid_threads : 0;
+  return ADF_OK;
+}
+
 int adf_set_barrier_wait(adf_solver* s, long long polls, int extra_arrivals) {
   if (!s) return fail(ADF_ERR_VALUE, "adf_set_barrier_wait: null solver");
   if (polls < 1 || extra_arrivals < 0) return fail(ADF_ERR_VALUE, "adf_set_barrier_wait: polls >= 1, extra >= 0");

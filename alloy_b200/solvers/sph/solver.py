@@ -443,6 +443,13 @@ class SolverDFSPH:
         launches one kernel per phase, at that priority. The results are the same bits either way."""
         _lib.check(self._lib.adf_set_persistent(self._h, int(bool(enable))), "persistent")
 
+    def solve_launch(self) -> dict[str, int]:
+        """The shape of the one-launch solves (include/alloy_dfsph.h adf_solve_launch): form (-1 when the solves take one
+        kernel per phase), blocks and threads."""
+        shape = np.zeros(3, np.int32)
+        _lib.check(self._lib.adf_solve_launch(self._h, shape.ctypes.data), "solve_launch")
+        return {"form": int(shape[0]), "blocks": int(shape[1]), "threads": int(shape[2])}
+
     def halo(self, mode: int = 1) -> None:
         """Item halos of the Jacobi iterations (include/alloy_dfsph.h adf_set_halo): 1 staged, 0 global gathers (the
         default, measured faster), -1 the autotuner times both forms for the acceleration and Jacobi kernels. Same

@@ -197,6 +197,10 @@ int adf_halo_stats(adf_solver* solver, int32_t* in_use, int64_t* stats, void* st
  * phase, each at that priority, whatever `enable` says (a captured step keeps the form of the stream it was captured
  * on, and is to be launched on streams of that priority). */
 int adf_set_persistent(adf_solver* solver, int enable);
+/* The shape of that launch, chosen at creation from the particles that are or can become liquid (host int32[3]): form
+ * (-1 none: one kernel per phase; 0 rows in shared memory, up to 256 particles per SM; 1 one deep block per SM; 2 two wide
+ * ones), blocks, threads of a block. For tests of each form. */
+int adf_solve_launch(const adf_solver* solver, int32_t* shape);
 /* Test hook of the bounded barrier waits: each wait polls at most `polls` times (ADF_BARRIER_POLLS by default, some
  * twenty seconds: long enough for blocks that have started to wait for the others behind another stream's kernels), and a
  * barrier waits for `extra_arrivals` more blocks than the grid has (default 0; any other value makes every wait run out,
