@@ -21,7 +21,7 @@ DEPENDS = SOURCES + [CSRC / "dfsph_kernels.cuh", CSRC / "dfsph_mlp.cuh", CSRC / 
                      CSRC / "dfsph_port.cuh", CSRC / "dfsph_skin.cuh", CSRC / "dfsph_group.cuh", CSRC / "dfsph_small.cuh",
                      PKG.parent / "include" / "alloy_dfsph.h"]
 # No -split-compile: it builds in a third of the time, but which code it makes differs from run to run (150 of 179 kernels
-# between two builds of one source; the slower one took 6 % to 8 % longer on large worlds and 17 % on a step of 2,016 particles).
+# between two builds of one source; the slower one took 4 % to 7 % longer on a million particles and 17 % on 2,016).
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-fmad=false", "-prec-div=true",
               "-prec-sqrt=true", "-ftz=false", "-std=c++17", "-Xcompiler", "-fPIC", "-shared"]
 

@@ -629,11 +629,10 @@ int set_stream(adf_solver* s, cudaStream_t st) {
 
 // Whether this solve runs as one cooperative launch (dfsph_group.cuh). Steps that time kernels (tuning, profiling), steps
 // on a stream of raised priority and staged item halos take the kernels one by one, and so does a solver told to
-// (adf_set_persistent 0). The launch was
-// the faster one at every size measured, or equal (four steps, one kernel per phase against one launch): 2,016
-// particles 1.26 against 0.84 ms, the 30k column 4.08 against 2.56, 123k 1.89 against 1.55, 250k 3.07 against 2.70, the
-// 1M dam break 9.30 against 8.76, 256 columns 24.1 against 20.9, 6 worlds 1.90 against 1.61, 160 worlds 17.6 against
-// 17.4, the pour's first 1,024 worlds 60.6 against 59.8.
+// (adf_set_persistent 0). Up to the line of setup_grid_solve the launch was the faster one at every size measured (four
+// steps, one kernel per phase against one launch): 2,016 particles 1.05 against 0.57 ms, the 30k column 3.89 against 2.40,
+// its tank 2.75 against 1.73, 123k 1.87 against 1.47, the 1M dam break 9.20 against 8.51, 256 columns 23.7 against 19.8, 160
+// worlds 17.2 against 16.9, the pour's first 256 worlds with the learned start 18.4 against 17.8.
 bool grid_solves(const adf_solver* s, const DevP& P) {
   if (P.n_chunks == 0 || s->W == 0 || s->prof_on || s->grid_blocks == 0 || s->raised) return false;
   if (s->persist == 1 && s->cg) return true;
@@ -719,10 +718,11 @@ bool step_in_one(const adf_solver* s, const DevP& P) {
 // per SM their rows fit the SMs' shared memory (dfsph_small.cuh). Above, a thread each while the device holds that many:
 // every SM gets an even share. Above that, the form that takes fewer rounds (dfsph_group.cuh), for the Jacobi up to
 // JACOBI_ROUNDS of the deep one: past those a launch per phase, dealt out block by block and tuned to the model, costs less
-// than its boundaries (a step, one launch against one per phase: 3.1M particles 6.16 against 6.40 ms, pour of 1,024 worlds
-// 13.49 against 13.83, 6.3M particles 12.26 against 12.27, batched 512 worlds 12.91 against 12.78, pour of 2,048 worlds 27.2
-// against 26.5, of 4,096 56.8 against 52.7). The CG, whose launches per phase cover converged worlds too, gains at every
-// size (2,048 worlds 33.3 against 37.5).
+// than its boundaries on many worlds. A step, one launch against one per phase, in turn on one solver: 3.1M particles 6.29
+// against 6.50 ms, batched 400 worlds 10.30 against 10.41, pour of 1,024 worlds 13.18 against 13.62, of 1,400 (6.0M) 17.83
+// against 18.24, batched 512 worlds (6.1M) 13.13 against 13.17; past the line pour of 2,048 worlds (8.6M) 26.23 against 26.12,
+// of 4,096 54.7 against 52.0, but one world of 6.3M 13.96 against 14.57. The CG, whose launches per phase cover converged
+// worlds too, gains at every size (pour of 2,048 worlds 33.7 against 38.2).
 constexpr long long JACOBI_ROUNDS = 40;
 int setup_grid_solve(adf_solver* s, int sph) {
   CK(cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, s->device));

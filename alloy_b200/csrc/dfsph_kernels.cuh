@@ -2817,7 +2817,8 @@ __global__ void __launch_bounds__(256) k_world_sum2(DevP P, int with_max) {
 // by one takes 40 of doubles (80 instructions of a pipe that serves a warp every other cycle, so 32 warps of an SM folding
 // two sums each kept it busy for 5 us). Here a lane gives half of the groups it still holds to its partner and takes the
 // partner's share of the other half, the same pairs added: 4 + 2 + 1 + 1 + 1, and 3 for the group sums. With a fold for each
-// SM before a second, four steps of the 30k column took 2,495 -> 2,307 us, of the 30k tank 1,658 -> 1,520.
+// SM before a second, four steps of the 30k column took 2,480 -> 2,401 us, of the 30k tank 1,780 -> 1,729, of 256 columns
+// 20.9 -> 20.4 ms.
 __device__ __forceinline__ double fold256_lanes(double (&s)[8]) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
@@ -2862,7 +2863,7 @@ __device__ __forceinline__ float warp_max(float v) {
 // Both sums are of the step's start (the warm starts change only with its end), so one pass takes all six terms, a chunk's
 // values loaded once and its six trees side by side: what bounds it is latency (118 warps at 30k particles). Term after term
 // in four launches and a fifth for the factor took 56 us of the 30k tank's step (cold); four steps there with the state
-// copied and the counters cleared in the sort's kernels too: 1,740 -> 1,658 us.
+// copied and the counters cleared in the sort's kernels too: 1,914 -> 1,780 us.
 constexpr int JIT_TERMS = 6;
 
 // The terms of particle i (caller's order), 0 unless liquid: flow (v_z, 1, v_x, v_y; solve_driver.py:40-51) and head

@@ -8,8 +8,8 @@
 // divergence), all gathers of a row in flight at once, instead of rows, positions and that value.
 //
 // A step of such a model is one launch after its rows and walls (k_small_step): density, both solves, XSPH and the finish
-// read the rows once. Against a launch for each: four steps of 2,016 particles 685 -> 624 us, of 8,000 with reports 1085
-// -> 1020, of the 30k column 2551 -> 2495, of the 30k tank 1964 -> 1910.
+// read the rows once. Against a launch for each: four steps of 2,016 particles 673 -> 615 us, of 8,000 with reports 1,074
+// -> 1,010, of the 30k column 2,563 -> 2,514, of the 30k tank 1,971 -> 1,914.
 //
 // What bounded these phases before: on 30,720 particles an acceleration or divergence phase took 7 to 9 us, 21 MB
 // through the L2 after every barrier's L1 invalidation, in eight dependent trips a thread.

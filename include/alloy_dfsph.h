@@ -139,9 +139,10 @@ int adf_step(adf_solver* solver, const float* q_in, const float* qd_in, float* q
              const float* f_ext, double dt, void* stream);
 
 /* Step execution mode. enable = 1 (default): adf_step replays a CUDA graph of the whole step (built on first use per
- * state-pointer set and dt; the pressure iterations are WHILE nodes, as wp.capture_while, solve_driver.py:186);
+ * state-pointer set and dt; pressure iterations of one kernel per phase are WHILE nodes, as wp.capture_while,
+ * solve_driver.py:186);
  * 0: the same kernels launched one by one with the iteration count read back on the host. A step enqueued on a
- * stream that the caller is capturing always joins that capture with WHILE nodes. */
+ * stream that the caller is capturing always joins that capture, in the same form. */
 int adf_set_graphs(adf_solver* solver, int enable);
 
 /* Autotuner (no counterpart in the reference; Warp picks its own launch shapes). enable = 1 (the default at creation):
@@ -150,11 +151,15 @@ int adf_set_graphs(adf_solver* solver, int enable);
  * Jacobi update, XSPH, list build) runs, times every candidate (threads per block {128, 256} x neighbour gathers in
  * flight {4, 8, 16}; for the list build 32 or 16 particles per warp) three times on that step's inputs and keeps the
  * fastest; it synchronises the stream while it does and
- * its results equal an ordinary step's bit for bit. 0: the default configuration (256 threads, 8 gathers). */
+ * its results equal an ordinary step's bit for bit. 0: the default configuration (256 threads, 8 gathers). What is
+ * tuned steers the kernels that are launched one by one: the list build always; density and factor and XSPH on models above
+ * 256 liquid particles per SM, in steps with a learned start or feature record and in adf_density_ratio and adf_prime; the
+ * other three in a learned start with its first sweep and where solves take one kernel per phase (adf_set_persistent below).
+ * The one-launch solves have a shape of their own (adf_solve_launch). */
 #define ADF_TUNE_KERNELS 6 /* density and factor, solve start, acceleration (and apply), Jacobi, XSPH, list build */
 int adf_set_autotune(adf_solver* solver, int enable);
 /* Pin one kernel's configuration (one of the tuner's candidates; for the list build block 128 and nb = particles per
- * warp, 32 or 16); the tuner then leaves it as set. */
+ * warp, 32 or 16); the tuner then leaves it as set, and it steers what the tuner's choice would. */
 int adf_set_tuned_config(adf_solver* solver, int kernel, int block, int nb);
 /* The configuration in use per tuned kernel (host [ADF_TUNE_KERNELS] each, any may be NULL): threads per block,
  * gathers in flight, and the winning trial's milliseconds (-1 if not tuned). */

@@ -1,9 +1,10 @@
 # SPDX-License-Identifier: Apache-2.0
-"""The persistent CG solve: each projected-CG pressure solve of a model of at most 131,072 particles runs as one
-cooperative launch whose phases (the bodies of the multi-launch path's kernels) are separated by grid-wide barriers
-with bounded waits (krylov.py:254-297 with the loop of solve_driver.py:121-186).
+"""A pressure solve as one cooperative launch, told to run so in every step (persistent(True)), with the projected CG: the
+phases of a solve are separated by grid-wide barriers with bounded waits (krylov.py:254-297 with the loop of
+solve_driver.py:121-186). These models are small enough for their rows in shared memory; test_gpu_grid_solve.py and
+test_gpu_grid_solve_worlds.py cover the other forms and the Jacobi.
 
-- bit for bit against the multi-launch path (positions, velocities, warm starts, per-world iterations and errors every
+- bit for bit against one kernel per phase (positions, velocities, warm starts, per-world iterations and errors every
   step) on a dam break in a tank of boundary particles, on uneven batched worlds with spouts (active sets change,
   worlds stop at different iterations), and on primed resting columns in box tanks (four wall slots per
   particle), each replayed as CUDA graphs and launched eagerly; the launches per step drop;
@@ -11,8 +12,8 @@ with bounded waits (krylov.py:254-297 with the loop of solve_driver.py:121-186).
   fails with ADF_ERR_STATE instead of returning results, and after the status is cleared the solver steps on and
   equals a fresh solver bit for bit (no GPU fault, no unbounded wait).
 
-The multi-launch path, the default, is the one the tests against the oracle run; test_gpu_jitter_rule.py runs the
-persistent one against the oracle as well.
+The tests against the oracle run what a new solver runs, one launch per solve after the tuning step; test_gpu_per_phase.py
+runs one kernel per phase against it.
 """
 
 from __future__ import annotations
@@ -109,7 +110,7 @@ def test_persistent_barrier_wait_expires_with_status(cuda):
     with pytest.raises(RuntimeError, match="grid-barrier wait"):
         sol.report()
     sol.clear_status()
-    sol.barrier_wait()  # the defaults: the grid's own blocks, about a second per wait
+    sol.barrier_wait()  # the defaults: the grid's own blocks, the library's limit
     # the failed step's results are invalid: both solvers go on from the model's state with the same warm starts
     a, b = sc.model.state(), sc.model.state()
     mine, theirs = sol.alloy_state_arrays(), ref.alloy_state_arrays()
